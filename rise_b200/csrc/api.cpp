@@ -152,7 +152,6 @@ cudaError_t PipelinedCast(rtb200_scene* s, const rtb200_ray* rays, int64_t n, vo
         if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_up[b], ctx->copy_in);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(ts[b], ctx->ev_up[b], 0);
         if (e == cudaSuccess && k >= 2) e = cudaStreamWaitEvent(ts[b], ctx->ev_down[b], 0);   // chunk k-2 downloaded
-        if (e == cudaSuccess) e = cudaMemsetAsync(counter[b], 0, sizeof(unsigned long long), ts[b]);
         if (e == cudaSuccess) e = trace(d_in, m, d_out, counter[b], ts[b]);
         if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_trace[b], ts[b]);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->copy_out, ctx->ev_trace[b], 0);

@@ -667,23 +667,25 @@ int TraceStackBound(const BuiltBVH& b)
     return bound;
 }
 
+GpuTri EncodeTriangle(const float* tri9, uint32_t prim, bool last)
+{
+    const float* s = tri9 + 9 * (size_t)prim;
+    const int32_t w = (int32_t)(prim | (last ? 0x80000000u : 0u));
+    return GpuTri{{{s[0], s[3], s[6]}, w}, {{s[1], s[4], s[7]}, w}, {{s[2], s[5], s[8]}, w}};
+}
+
 void EncodeTriangles(const float* tri9, const BuiltBVH& b, std::vector<GpuTri>& out)
 {
     out.resize(b.prims.size());
-    for (size_t i = 0; i < b.prims.size(); ++i) {
-        const uint32_t p = b.prims[i];
-        const float* s = tri9 + 9 * (size_t)p;
-        GpuTri& t = out[i];
-        for (int k = 0; k < 3; ++k) { t.v0[k] = s[k]; t.v1[k] = s[3 + k]; t.v2[k] = s[6 + k]; }
-        std::memcpy(&t.v0[3], &p, 4);
-        t.v1[3] = 0.0f;
-        t.v2[3] = 0.0f;
-    }
-    // Mark the last triangle of every leaf (v1.w = 1) so the traversal can
-    // walk a leaf from its first slot without a separate count.
+    for (size_t i = 0; i < b.prims.size(); ++i) out[i] = EncodeTriangle(tri9, b.prims[i], false);
+    // Flag the last triangle of every leaf so the traversal can walk a leaf
+    // from its first slot without a separate count.
     for (const Node4& n : b.nodes4)
         for (int i = 0; i < n.nchild; ++i)
-            if (n.count[i] > 0) out[(size_t)n.child[i] + n.count[i] - 1].v1[3] = 1.0f;
+            if (n.count[i] > 0) {
+                const size_t at = (size_t)n.child[i] + n.count[i] - 1;
+                out[at] = EncodeTriangle(tri9, b.prims[at], true);
+            }
 }
 
 }  // namespace rtb200

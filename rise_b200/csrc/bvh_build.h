@@ -77,8 +77,8 @@ void MergeMeshBVHs(const std::vector<MeshBVH2>& meshes, BuiltBVH& out);
 // FP32 wide node: 4 child boxes as SoA float4 + child links, 128 bytes.
 // child[i] >= 0: internal node index; child[i] == INT32_MIN: empty slot;
 // other child[i] < 0: a leaf whose first triangle (in leaf order) is
-// ~child[i], holding count[i] triangles (the last one carries
-// GpuTri::v1[3] == 1).  The traversal reads the first 112 bytes only (empty
+// ~child[i], holding count[i] triangles (the last one is flagged in
+// GpuTri).  The traversal reads the first 112 bytes only (empty
 // slots are known from the link); count[i] (-1 for an empty slot) is kept
 // for the host's view of the node.
 struct alignas(16) GpuNode4 {
@@ -121,11 +121,16 @@ static_assert(sizeof(HNode4) == 64, "HNode4 must be 64 bytes");
 float HalfToFloat(uint16_t h);
 uint16_t FloatToHalfDirected(float x, int dir);
 
-// One triangle in leaf order: v0.w carries the input triangle index.
+// One triangle in leaf order, a row per coordinate: the values of v0, v1 and
+// v2, then the input triangle index (31 bits) under the flag of a leaf's last
+// triangle, repeated in every row.  A ray reads the rows in the order of its
+// permuted axes, so the watertight test needs no per-triangle axis selects.
+constexpr int kTriIndexMask = 0x7fffffff;
 struct alignas(16) GpuTri {
-    float v0[4];
-    float v1[4];
-    float v2[4];
+    struct {
+        float v[3];
+        int32_t w;
+    } x, y, z;
 };
 static_assert(sizeof(GpuTri) == 48, "GpuTri must be 48 bytes");
 
@@ -159,6 +164,7 @@ void EncodeGpuNodes(const BuiltBVH& b, std::vector<GpuNode4>& out);
 void EncodeQuantNodes(const BuiltBVH& b, std::vector<QNode4>& out);
 void EncodeHalfNodes(const BuiltBVH& b, std::vector<HNode4>& out);
 void EncodeTriangles(const float* tri9, const BuiltBVH& b, std::vector<GpuTri>& out);
+GpuTri EncodeTriangle(const float* tri9, uint32_t prim, bool last);
 
 // Upper bound on the traversal stack depth of the BVH4: the largest sum of
 // (children - 1) over the internal nodes of one root-to-node path.  A

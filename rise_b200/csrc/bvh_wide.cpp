@@ -205,16 +205,9 @@ bool EncodeWideNodes(const BuiltBVH& b, std::vector<WNode8>& nodes, std::vector<
 
 void EncodeWideTriangles(const float* tri9, const std::vector<uint32_t>& prims, std::vector<GpuTri>& out)
 {
+    // Every triangle is its own run: no leaf walk continues past it.
     out.resize(prims.size());
-    for (size_t i = 0; i < prims.size(); ++i) {
-        const uint32_t p = prims[i];
-        const float* s = tri9 + 9 * (size_t)p;
-        GpuTri& t = out[i];
-        for (int k = 0; k < 3; ++k) { t.v0[k] = s[k]; t.v1[k] = s[3 + k]; t.v2[k] = s[6 + k]; }
-        std::memcpy(&t.v0[3], &p, 4);
-        t.v1[3] = 1.0f;   // every triangle is its own run: no leaf walk continues past it
-        t.v2[3] = 0.0f;
-    }
+    for (size_t i = 0; i < prims.size(); ++i) out[i] = EncodeTriangle(tri9, prims[i], true);
 }
 
 }  // namespace rtb200

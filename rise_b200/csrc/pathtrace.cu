@@ -403,12 +403,13 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
     int spill[SPILL ? kTraceSpill : 1];
     const TraceStack stk{sstack + threadIdx.x, spill};
     const long long n = Q.cnt[kCntActive];
-    WarpFeed feed{0ull, 0ull, false};
+    const int chunk = FeedChunk((unsigned long long)n, (gridDim.x * blockDim.x) >> 5);
+    WarpFeed feed = FeedStart((unsigned long long)n, chunk);
     TraceState s;
     long long qi = -1;
     int slot = -1;
     for (;;) {
-        const long long got = FeedTake(feed, qi < 0, (unsigned long long)n, Q.trace_ctr);
+        const long long got = FeedTake(feed, qi < 0, (unsigned long long)n, chunk, Q.trace_ctr);
         if (got >= 0) {
             qi = got;
             slot = Q.active[qi];
@@ -445,11 +446,12 @@ KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
     int spill[SPILL ? kTraceSpill : 1];
     const TraceStack stk{sstack + threadIdx.x, spill};
     const long long n = Q.cnt[kCntShadow];
-    WarpFeed feed{0ull, 0ull, false};
+    const int chunk = FeedChunk((unsigned long long)n, (gridDim.x * blockDim.x) >> 5);
+    WarpFeed feed = FeedStart((unsigned long long)n, chunk);
     TraceState s;
     long long qi = -1;
     for (;;) {
-        const long long got = FeedTake(feed, qi < 0, (unsigned long long)n, Q.trace_ctr + 1);
+        const long long got = FeedTake(feed, qi < 0, (unsigned long long)n, chunk, Q.trace_ctr + 1);
         if (got >= 0) {
             qi = got;
             const ShadowEntry e = Q.shadow[qi];
@@ -641,8 +643,8 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
             }
             const float t = h.x;
             const V3 p = xyz(ro) + d * t;
-            const float* tb = reinterpret_cast<const float*>(S.tris + hslot);
-            const float4 A = ldg4(tb), B = ldg4(tb + 4), C = ldg4(tb + 8);
+            float4 A, B, C;
+            LoadVertices(S.tris, hslot, A, B, C);
             const V3 nface = normalize(cross(xyz(B) - xyz(A), xyz(C) - xyz(A)));
             const PtTriAttr at = S.attr[hslot];
             const int mi = at.mat & kAttrMatMask;

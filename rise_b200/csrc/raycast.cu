@@ -31,16 +31,16 @@ template <class NodeT, bool ANY, bool SPILL>
 __global__ void __launch_bounds__(kTraceBlock, 8)
 KTrace(const NodeT* __restrict__ nodes, const GpuTri* __restrict__ tris,
        const rtb200_ray* __restrict__ rays, long long n, int ntri, rtb200_hit* __restrict__ hits,
-       uint8_t* __restrict__ occ, unsigned long long* counter, unsigned* err)
+       uint8_t* __restrict__ occ, int chunk, unsigned long long* counter, unsigned* err)
 {
     __shared__ int sstack[kTraceStack * kTraceBlock];
     int spill[SPILL ? kTraceSpill : 1];
     const TraceStack stk{sstack + threadIdx.x, spill};
-    WarpFeed feed{0ull, 0ull, false};
+    WarpFeed feed = FeedStart((unsigned long long)n, chunk);
     TraceState s;
     long long ray = -1;
     for (;;) {
-        const long long got = FeedTake(feed, ray < 0, (unsigned long long)n, counter);
+        const long long got = FeedTake(feed, ray < 0, (unsigned long long)n, chunk, counter);
         if (got >= 0) {
             ray = got;
             StartRay(s, LoadRay(rays, ray));
@@ -52,10 +52,11 @@ KTrace(const NodeT* __restrict__ nodes, const GpuTri* __restrict__ tris,
             } else {
                 float4 out;
                 if (s.bestSlot >= 0) {
-                    const float* tb = reinterpret_cast<const float*>(tris + s.bestSlot);
-                    const float4 A = ldg4(tb), B = ldg4(tb + 4), C = ldg4(tb + 8);
-                    out.x = (float)RefineT(s.p.o, s.d, A, B, C);
-                    out.y = A.w;  // input triangle index (bit pattern)
+                    float4 A, B, C;
+                    LoadVertices(tris, s.bestSlot, A, B, C);
+                    const Ray r = LoadRay(rays, ray);   // again: the direction is not kept during the walk
+                    out.x = (float)RefineT(r.o, r.d, A, B, C);
+                    out.y = __int_as_float(TriIndex(tris, s.bestSlot));
                     out.z = s.ba;
                     out.w = s.bb;
                 } else {
@@ -76,16 +77,16 @@ constexpr int kW8Budget = 16;
 template <bool ANY>
 __global__ void __launch_bounds__(kTraceBlock, 8)
 KTraceW8(const WNode8* __restrict__ nodes, const GpuTri* __restrict__ tris, const rtb200_ray* __restrict__ rays,
-         long long n, rtb200_hit* __restrict__ hits, uint8_t* __restrict__ occ, unsigned long long* counter,
-         unsigned* err)
+         long long n, rtb200_hit* __restrict__ hits, uint8_t* __restrict__ occ, int chunk,
+         unsigned long long* counter, unsigned* err)
 {
     __shared__ uint2 sstack[kW8Stack * kTraceBlock];
     uint2* stk = sstack + threadIdx.x;
-    WarpFeed feed{0ull, 0ull, false};
+    WarpFeed feed = FeedStart((unsigned long long)n, chunk);
     W8State s;
     long long ray = -1;
     for (;;) {
-        const long long got = FeedTake(feed, ray < 0, (unsigned long long)n, counter);
+        const long long got = FeedTake(feed, ray < 0, (unsigned long long)n, chunk, counter);
         if (got >= 0) {
             ray = got;
             StartRayW8(s, LoadRay(rays, ray));
@@ -97,10 +98,10 @@ KTraceW8(const WNode8* __restrict__ nodes, const GpuTri* __restrict__ tris, cons
             } else {
                 float4 out;
                 if (s.bestSlot >= 0) {
-                    const float* tb = reinterpret_cast<const float*>(tris + s.bestSlot);
-                    const float4 A = ldg4(tb), B = ldg4(tb + 4), C = ldg4(tb + 8);
+                    float4 A, B, C;
+                    LoadVertices(tris, s.bestSlot, A, B, C);
                     out.x = (float)RefineT(s.p.o, s.d, A, B, C);
-                    out.y = A.w;
+                    out.y = __int_as_float(TriIndex(tris, s.bestSlot));
                     out.z = s.ba;
                     out.w = s.bb;
                 } else {
@@ -123,23 +124,44 @@ int GridFor(K kernel, int num_sms)
 }
 
 // One launch over `n` rays with the work counter and error word given.  The
-// grid is the kernel's occupancy times the SM count, cached per instantiation
-// and device (devices of one process may differ).
+// full grid is the kernel's occupancy times the SM count, cached per
+// instantiation and device (devices of one process may differ).  Batches of
+// up to 32 rays per resident warp launch only the warps that get a ray and
+// never touch the counter; larger ones clear it first.
 constexpr int kGridDevices = 64;
 
-template <class NodeT, bool ANY, bool SPILL>
-void Launch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n, rtb200_hit* hits, uint8_t* occ,
-            unsigned long long* counter, unsigned* err, cudaStream_t stream)
+template <class K>
+cudaError_t PlanFeed(K kernel, std::atomic<int>* grids, const rtb200_ctx* ctx, int64_t n, unsigned long long* counter,
+                     cudaStream_t stream, int& grid, int& chunk)
 {
-    static std::atomic<int> grids[kGridDevices];
-    const int dev = s->ctx->device;
-    int grid = (dev >= 0 && dev < kGridDevices) ? grids[dev].load(std::memory_order_relaxed) : 0;
+    constexpr int kWarps = kTraceBlock / 32;
+    const int dev = ctx->device;
+    grid = (dev >= 0 && dev < kGridDevices) ? grids[dev].load(std::memory_order_relaxed) : 0;
     if (!grid) {
-        grid = GridFor(KTrace<NodeT, ANY, SPILL>, s->ctx->num_sms);
+        grid = GridFor(kernel, ctx->num_sms);
         if (dev >= 0 && dev < kGridDevices) grids[dev].store(grid, std::memory_order_relaxed);
     }
+    chunk = FeedChunk((unsigned long long)n, (unsigned long long)grid * kWarps);
+    const int64_t blocks = ((n + chunk - 1) / chunk + kWarps - 1) / kWarps;
+    if (blocks <= grid) {
+        grid = (int)blocks;
+        return cudaSuccess;
+    }
+    return cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
+}
+
+template <class NodeT, bool ANY, bool SPILL>
+cudaError_t Launch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n, rtb200_hit* hits, uint8_t* occ,
+                   unsigned long long* counter, unsigned* err, cudaStream_t stream)
+{
+    static std::atomic<int> grids[kGridDevices];
+    int grid, chunk;
+    const cudaError_t e = PlanFeed(KTrace<NodeT, ANY, SPILL>, grids, s->ctx, n, counter, stream, grid, chunk);
+    if (e != cudaSuccess) return e;
     KTrace<NodeT, ANY, SPILL><<<grid, kTraceBlock, 0, stream>>>((const NodeT*)s->d_nodes, s->d_tris, d_rays, n,
-                                                                (int)s->tri_material.size(), hits, occ, counter, err);
+                                                                (int)s->tri_material.size(), hits, occ, chunk, counter,
+                                                                err);
+    return cudaGetLastError();
 }
 
 template <bool ANY>
@@ -150,25 +172,21 @@ cudaError_t Dispatch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n,
     const bool spill = s->stack_bound > kTraceStack;
     if (s->layout == RTB200_BVH_W8) {
         static std::atomic<int> grids[kGridDevices];
-        const int dev = s->ctx->device;
-        int grid = (dev >= 0 && dev < kGridDevices) ? grids[dev].load(std::memory_order_relaxed) : 0;
-        if (!grid) {
-            grid = GridFor(KTraceW8<ANY>, s->ctx->num_sms);
-            if (dev >= 0 && dev < kGridDevices) grids[dev].store(grid, std::memory_order_relaxed);
-        }
+        int grid, chunk;
+        const cudaError_t e = PlanFeed(KTraceW8<ANY>, grids, s->ctx, n, counter, stream, grid, chunk);
+        if (e != cudaSuccess) return e;
         KTraceW8<ANY><<<grid, kTraceBlock, 0, stream>>>((const WNode8*)s->d_nodes, s->d_tris, d_rays, n, hits, occ,
-                                                        counter, err);
-    } else if (s->layout == RTB200_BVH_Q8) {
-        if (spill) Launch<QNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream);
-        else Launch<QNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
-    } else if (s->layout == RTB200_BVH_F16) {
-        if (spill) Launch<HNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream);
-        else Launch<HNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
-    } else {
-        if (spill) Launch<GpuNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream);
-        else Launch<GpuNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
+                                                        chunk, counter, err);
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
+    if (s->layout == RTB200_BVH_Q8)
+        return spill ? Launch<QNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream)
+                     : Launch<QNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
+    if (s->layout == RTB200_BVH_F16)
+        return spill ? Launch<HNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream)
+                     : Launch<HNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
+    return spill ? Launch<GpuNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream)
+                 : Launch<GpuNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
 }
 
 }  // namespace
@@ -176,9 +194,6 @@ cudaError_t Dispatch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n,
 cudaError_t LaunchCastClosest(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n,
                               rtb200_hit* d_hits, cudaStream_t stream)
 {
-    if (n <= 0) return cudaSuccess;
-    const cudaError_t e = cudaMemsetAsync(s->d_counter, 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
     return Dispatch<false>(s, d_rays, n, d_hits, nullptr, s->d_counter, s->d_err, stream);
 }
 
@@ -198,9 +213,6 @@ cudaError_t LaunchCastAnyScratch(const rtb200_scene* s, const rtb200_ray* d_rays
 cudaError_t LaunchCastAny(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n,
                           uint8_t* d_occ, cudaStream_t stream)
 {
-    if (n <= 0) return cudaSuccess;
-    const cudaError_t e = cudaMemsetAsync(s->d_counter, 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
     return Dispatch<true>(s, d_rays, n, nullptr, d_occ, s->d_counter, s->d_err, stream);
 }
 
