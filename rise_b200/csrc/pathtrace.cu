@@ -392,7 +392,7 @@ KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int assign)
 // hit stores the leaf-order triangle slot for shading.
 // UNIFORM: every job shares the scene `us` (kernel argument, no per-path
 // lookup of the job's scene).
-template <class NodeT, bool SPILL, bool UNIFORM>
+template <class NodeT, bool SPILL, bool UNIFORM, bool COOP>
 __global__ void __launch_bounds__(kTraceBlock, 8)
 KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
 {
@@ -402,14 +402,15 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
     __shared__ int sstack[kTraceStack * kTraceBlock];
     int spill[SPILL ? kTraceSpill : 1];
     const TraceStack stk{sstack + threadIdx.x, spill};
-    const long long n = Q.cnt[kCntActive];
-    const int chunk = FeedChunk((unsigned long long)n, (gridDim.x * blockDim.x) >> 5);
-    WarpFeed feed = FeedStart((unsigned long long)n, chunk);
+    const unsigned n = (unsigned)Q.cnt[kCntActive];
+    const unsigned chunk = FeedChunk(n, (gridDim.x * blockDim.x) >> 5);
+    WarpFeed feed = FeedStart(n, chunk);
     TraceState s;
-    long long qi = -1;
+    if (COOP) s.sp = 0;
+    int qi = -1;
     int slot = -1;
     for (;;) {
-        const long long got = FeedTake(feed, qi < 0, (unsigned long long)n, chunk, Q.trace_ctr);
+        const int got = FeedTake(feed, qi < 0, n, chunk, (unsigned*)Q.trace_ctr);
         if (got >= 0) {
             qi = got;
             slot = Q.active[qi];
@@ -425,17 +426,33 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
             r.d[0] = d.x; r.d[1] = d.y; r.d[2] = d.z; r.tmax = d.w;
             StartRay(s, r);
         }
-        if (__all_sync(kFull, qi < 0)) break;
+        const unsigned live = __ballot_sync(kFull, qi >= 0);
+        if (!live) return;
+        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, live)) break;
         if (qi >= 0 && TraceRound<NodeT, false, SPILL, kPathLeaves>(s, nodes, tris, ntri, stk, Q.err)) {
             P.hit[slot] = make_float4(s.best, __int_as_float(s.bestSlot), s.ba, s.bb);
             qi = -1;
         }
     }
+    if (COOP) {
+        CoopFinish<NodeT, false, SPILL>(s, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
+        if (qi >= 0) P.hit[slot] = make_float4(s.best, __int_as_float(s.bestSlot), s.ba, s.bb);
+    }
+}
+
+// Adds an unoccluded shadow entry's contribution to its path's radiance.
+__device__ __forceinline__ void AddShadow(const PtPaths& P, const ShadowEntry& e)
+{
+    float* l = reinterpret_cast<float*>(P.L + __float_as_int(e.d.w));
+    if (e.c.x != 0.0f) atomicAdd(l + 0, e.c.x);
+    if (e.c.y != 0.0f) atomicAdd(l + 1, e.c.y);
+    if (e.c.z != 0.0f) atomicAdd(l + 2, e.c.z);
+    if (e.c.w != 0.0f) atomicAdd(l + 3, e.c.w);
 }
 
 // Any hit for the shadow-ray queue; unoccluded entries add their
 // contribution to the path's radiance.
-template <class NodeT, bool SPILL, bool UNIFORM>
+template <class NodeT, bool SPILL, bool UNIFORM, bool COOP>
 __global__ void __launch_bounds__(kTraceBlock, 8)
 KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
 {
@@ -445,13 +462,14 @@ KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
     __shared__ int sstack[kTraceStack * kTraceBlock];
     int spill[SPILL ? kTraceSpill : 1];
     const TraceStack stk{sstack + threadIdx.x, spill};
-    const long long n = Q.cnt[kCntShadow];
-    const int chunk = FeedChunk((unsigned long long)n, (gridDim.x * blockDim.x) >> 5);
-    WarpFeed feed = FeedStart((unsigned long long)n, chunk);
+    const unsigned n = (unsigned)Q.cnt[kCntShadow];
+    const unsigned chunk = FeedChunk(n, (gridDim.x * blockDim.x) >> 5);
+    WarpFeed feed = FeedStart(n, chunk);
     TraceState s;
-    long long qi = -1;
+    if (COOP) s.sp = 0;
+    int qi = -1;
     for (;;) {
-        const long long got = FeedTake(feed, qi < 0, (unsigned long long)n, chunk, Q.trace_ctr + 1);
+        const int got = FeedTake(feed, qi < 0, n, chunk, (unsigned*)(Q.trace_ctr + 1));
         if (got >= 0) {
             qi = got;
             const ShadowEntry e = Q.shadow[qi];
@@ -466,19 +484,17 @@ KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
             r.d[0] = e.d.x; r.d[1] = e.d.y; r.d[2] = e.d.z; r.tmax = e.o.w;
             StartRay(s, r);
         }
-        if (__all_sync(kFull, qi < 0)) break;
+        const unsigned live = __ballot_sync(kFull, qi >= 0);
+        if (!live) return;
+        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, live)) break;
         if (qi >= 0 && TraceRound<NodeT, true, SPILL, kPathLeaves>(s, nodes, tris, ntri, stk, Q.err)) {
-            if (s.bestSlot < 0) {
-                const ShadowEntry& e = Q.shadow[qi];
-                const int slot = __float_as_int(e.d.w);
-                float* l = reinterpret_cast<float*>(P.L + slot);
-                if (e.c.x != 0.0f) atomicAdd(l + 0, e.c.x);
-                if (e.c.y != 0.0f) atomicAdd(l + 1, e.c.y);
-                if (e.c.z != 0.0f) atomicAdd(l + 2, e.c.z);
-                if (e.c.w != 0.0f) atomicAdd(l + 3, e.c.w);
-            }
+            if (s.bestSlot < 0) AddShadow(P, Q.shadow[qi]);
             qi = -1;
         }
+    }
+    if (COOP) {
+        CoopFinish<NodeT, true, SPILL>(s, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
+        if (qi >= 0 && s.bestSlot < 0) AddShadow(P, Q.shadow[qi]);
     }
 }
 
@@ -1227,29 +1243,36 @@ int TraceGrid(K kernel, int sms)
 
 // Extension kernel (closest hits of the path queue) when `extend`, else the
 // connection kernel (shadow rays); grids cached per instantiation.
-template <class NodeT, bool SPILL, bool UNIFORM>
+template <class NodeT, bool SPILL, bool UNIFORM, bool COOP>
 void LaunchTraceKernels(const PtLaunch& L, cudaStream_t st, bool extend)
 {
     if (extend) {
         static int g = 0;
-        if (!g) g = TraceGrid(KExtend<NodeT, SPILL, UNIFORM>, L.sms);
-        KExtend<NodeT, SPILL, UNIFORM><<<g, kTraceBlock, 0, st>>>(L.jobs, L.paths, L.queues, L.scene);
+        if (!g) g = TraceGrid(KExtend<NodeT, SPILL, UNIFORM, COOP>, L.sms);
+        KExtend<NodeT, SPILL, UNIFORM, COOP><<<g, kTraceBlock, 0, st>>>(L.jobs, L.paths, L.queues, L.scene);
     } else {
         static int g = 0;
-        if (!g) g = TraceGrid(KConnect<NodeT, SPILL, UNIFORM>, L.sms);
-        KConnect<NodeT, SPILL, UNIFORM><<<g, kTraceBlock, 0, st>>>(L.jobs, L.paths, L.queues, L.scene);
+        if (!g) g = TraceGrid(KConnect<NodeT, SPILL, UNIFORM, COOP>, L.sms);
+        KConnect<NodeT, SPILL, UNIFORM, COOP><<<g, kTraceBlock, 0, st>>>(L.jobs, L.paths, L.queues, L.scene);
     }
+}
+
+template <class NodeT, bool SPILL, bool UNIFORM>
+void LaunchTraceCoop(const PtLaunch& L, cudaStream_t st, bool extend)
+{
+    if (L.coop) LaunchTraceKernels<NodeT, SPILL, UNIFORM, true>(L, st, extend);
+    else LaunchTraceKernels<NodeT, SPILL, UNIFORM, false>(L, st, extend);
 }
 
 template <class NodeT>
 void LaunchTrace(const PtLaunch& L, cudaStream_t st, bool extend)
 {
     if (L.spill) {
-        if (L.uniform) LaunchTraceKernels<NodeT, true, true>(L, st, extend);
-        else LaunchTraceKernels<NodeT, true, false>(L, st, extend);
+        if (L.uniform) LaunchTraceCoop<NodeT, true, true>(L, st, extend);
+        else LaunchTraceCoop<NodeT, true, false>(L, st, extend);
     } else {
-        if (L.uniform) LaunchTraceKernels<NodeT, false, true>(L, st, extend);
-        else LaunchTraceKernels<NodeT, false, false>(L, st, extend);
+        if (L.uniform) LaunchTraceCoop<NodeT, false, true>(L, st, extend);
+        else LaunchTraceCoop<NodeT, false, false>(L, st, extend);
     }
 }
 

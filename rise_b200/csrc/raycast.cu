@@ -6,6 +6,7 @@
 // busy on the long tail of incoherent rays.  Rays are read as two 16-byte
 // vector loads and hits written as one 16-byte store; the traversal stack
 // lives in shared memory ([depth][thread], conflict-free).
+#include <algorithm>
 #include <atomic>
 
 #include "core.h"
@@ -13,7 +14,7 @@
 
 namespace rtb200 {
 
-__device__ __forceinline__ Ray LoadRay(const rtb200_ray* rays, long long i)
+__device__ __forceinline__ Ray LoadRay(const rtb200_ray* rays, int i)
 {
     const float4 a = ldg4(rays + i);
     const float4 b = ldg4(reinterpret_cast<const float*>(rays + i) + 4);
@@ -27,45 +28,63 @@ __device__ __forceinline__ Ray LoadRay(const rtb200_ray* rays, long long i)
 // best for both closest and any hit on incoherent rays).
 constexpr int kCastLeaves = 2;
 
-template <class NodeT, bool ANY, bool SPILL>
+// Stores a finished ray's answer: its occlusion flag, or its closest hit with
+// the distance re-measured in FP64.  The ray is read again: its direction is
+// not kept during the walk.
+template <bool ANY>
+__device__ __forceinline__ void StoreAnswer(const TraceState& s, const GpuTri* __restrict__ tris,
+                                            const rtb200_ray* __restrict__ rays, int ray,
+                                            rtb200_hit* __restrict__ hits, uint8_t* __restrict__ occ)
+{
+    if (ANY) {
+        occ[ray] = s.bestSlot >= 0 ? 1 : 0;
+        return;
+    }
+    float4 out = make_float4(-1.0f, __int_as_float(-1), 0.0f, 0.0f);
+    if (s.bestSlot >= 0) {
+        float4 A, B, C;
+        LoadVertices(tris, s.bestSlot, A, B, C);
+        const Ray r = LoadRay(rays, ray);
+        out.x = (float)RefineT(r.o, r.d, A, B, C);
+        out.y = __int_as_float(TriIndex(tris, s.bestSlot));
+        out.z = s.ba;
+        out.w = s.bb;
+    }
+    *reinterpret_cast<float4*>(hits + ray) = out;
+}
+
+// COOP: the last rays of a warp are finished by all its lanes (CoopFinish);
+// the rule for its use is in Launch.
+template <class NodeT, bool ANY, bool SPILL, bool COOP>
 __global__ void __launch_bounds__(kTraceBlock, 8)
 KTrace(const NodeT* __restrict__ nodes, const GpuTri* __restrict__ tris,
-       const rtb200_ray* __restrict__ rays, long long n, int ntri, rtb200_hit* __restrict__ hits,
-       uint8_t* __restrict__ occ, int chunk, unsigned long long* counter, unsigned* err)
+       const rtb200_ray* __restrict__ rays, unsigned n, int ntri, rtb200_hit* __restrict__ hits,
+       uint8_t* __restrict__ occ, unsigned chunk, unsigned* counter, unsigned* err)
 {
     __shared__ int sstack[kTraceStack * kTraceBlock];
     int spill[SPILL ? kTraceSpill : 1];
     const TraceStack stk{sstack + threadIdx.x, spill};
-    WarpFeed feed = FeedStart((unsigned long long)n, chunk);
+    WarpFeed feed = FeedStart(n, chunk);
     TraceState s;
-    long long ray = -1;
+    if (COOP) s.sp = 0;
+    int ray = -1;
     for (;;) {
-        const long long got = FeedTake(feed, ray < 0, (unsigned long long)n, chunk, counter);
+        const int got = FeedTake(feed, ray < 0, n, chunk, counter);
         if (got >= 0) {
             ray = got;
             StartRay(s, LoadRay(rays, ray));
         }
-        if (__all_sync(kFull, ray < 0)) break;
+        const unsigned live = __ballot_sync(kFull, ray >= 0);
+        if (!live) return;
+        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, live)) break;
         if (ray >= 0 && TraceRound<NodeT, ANY, SPILL, kCastLeaves>(s, nodes, tris, ntri, stk, err)) {
-            if (ANY) {
-                occ[ray] = s.bestSlot >= 0 ? 1 : 0;
-            } else {
-                float4 out;
-                if (s.bestSlot >= 0) {
-                    float4 A, B, C;
-                    LoadVertices(tris, s.bestSlot, A, B, C);
-                    const Ray r = LoadRay(rays, ray);   // again: the direction is not kept during the walk
-                    out.x = (float)RefineT(r.o, r.d, A, B, C);
-                    out.y = __int_as_float(TriIndex(tris, s.bestSlot));
-                    out.z = s.ba;
-                    out.w = s.bb;
-                } else {
-                    out = make_float4(-1.0f, __int_as_float(-1), 0.0f, 0.0f);
-                }
-                *reinterpret_cast<float4*>(hits + ray) = out;
-            }
+            StoreAnswer<ANY>(s, tris, rays, ray, hits, occ);
             ray = -1;
         }
+    }
+    if (COOP) {
+        CoopFinish<NodeT, ANY, SPILL>(s, ray >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), err);
+        if (ray >= 0) StoreAnswer<ANY>(s, tris, rays, ray, hits, occ);
     }
 }
 
@@ -77,16 +96,16 @@ constexpr int kW8Budget = 16;
 template <bool ANY>
 __global__ void __launch_bounds__(kTraceBlock, 8)
 KTraceW8(const WNode8* __restrict__ nodes, const GpuTri* __restrict__ tris, const rtb200_ray* __restrict__ rays,
-         long long n, rtb200_hit* __restrict__ hits, uint8_t* __restrict__ occ, int chunk,
-         unsigned long long* counter, unsigned* err)
+         unsigned n, rtb200_hit* __restrict__ hits, uint8_t* __restrict__ occ, unsigned chunk, unsigned* counter,
+         unsigned* err)
 {
     __shared__ uint2 sstack[kW8Stack * kTraceBlock];
     uint2* stk = sstack + threadIdx.x;
-    WarpFeed feed = FeedStart((unsigned long long)n, chunk);
+    WarpFeed feed = FeedStart(n, chunk);
     W8State s;
-    long long ray = -1;
+    int ray = -1;
     for (;;) {
-        const long long got = FeedTake(feed, ray < 0, (unsigned long long)n, chunk, counter);
+        const int got = FeedTake(feed, ray < 0, n, chunk, counter);
         if (got >= 0) {
             ray = got;
             StartRayW8(s, LoadRay(rays, ray));
@@ -131,62 +150,88 @@ int GridFor(K kernel, int num_sms)
 constexpr int kGridDevices = 64;
 
 template <class K>
-cudaError_t PlanFeed(K kernel, std::atomic<int>* grids, const rtb200_ctx* ctx, int64_t n, unsigned long long* counter,
-                     cudaStream_t stream, int& grid, int& chunk)
+cudaError_t PlanFeed(K kernel, std::atomic<int>* grids, const rtb200_ctx* ctx, unsigned n, unsigned* counter,
+                     cudaStream_t stream, int& grid, unsigned& chunk)
 {
-    constexpr int kWarps = kTraceBlock / 32;
+    constexpr unsigned kWarps = kTraceBlock / 32;
     const int dev = ctx->device;
     grid = (dev >= 0 && dev < kGridDevices) ? grids[dev].load(std::memory_order_relaxed) : 0;
     if (!grid) {
         grid = GridFor(kernel, ctx->num_sms);
         if (dev >= 0 && dev < kGridDevices) grids[dev].store(grid, std::memory_order_relaxed);
     }
-    chunk = FeedChunk((unsigned long long)n, (unsigned long long)grid * kWarps);
-    const int64_t blocks = ((n + chunk - 1) / chunk + kWarps - 1) / kWarps;
-    if (blocks <= grid) {
+    chunk = FeedChunk(n, (unsigned)grid * kWarps);
+    const unsigned blocks = ((n + chunk - 1) / chunk + kWarps - 1) / kWarps;
+    if (blocks <= (unsigned)grid) {
         grid = (int)blocks;
         return cudaSuccess;
     }
-    return cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
+    return cudaMemsetAsync(counter, 0, sizeof(unsigned), stream);
 }
 
-template <class NodeT, bool ANY, bool SPILL>
-cudaError_t Launch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n, rtb200_hit* hits, uint8_t* occ,
-                   unsigned long long* counter, unsigned* err, cudaStream_t stream)
+// Batches of up to this many rays per SM (the resident warps' first 128 rays
+// each) use the kernels whose warps finish their last rays together.  Without
+// and with (binary16 boxes, 300k-triangle soup): 20,000 rays 164 and 87 us,
+// 100,003 255 and 167, 500,000 483 and 436, 1,000,000 (1M triangles) 916 and
+// 907; at 4,194,304 the last rays no longer count and the joint walk's code
+// costs the lane walk registers (3340 and 3505 us).
+constexpr unsigned kCoopBatchPerSm = 4096;
+
+template <class NodeT, bool ANY, bool SPILL, bool COOP>
+cudaError_t LaunchKernel(const rtb200_scene* s, const rtb200_ray* d_rays, unsigned n, rtb200_hit* hits, uint8_t* occ,
+                         unsigned* counter, unsigned* err, cudaStream_t stream)
 {
     static std::atomic<int> grids[kGridDevices];
-    int grid, chunk;
-    const cudaError_t e = PlanFeed(KTrace<NodeT, ANY, SPILL>, grids, s->ctx, n, counter, stream, grid, chunk);
+    int grid;
+    unsigned chunk;
+    const cudaError_t e = PlanFeed(KTrace<NodeT, ANY, SPILL, COOP>, grids, s->ctx, n, counter, stream, grid, chunk);
     if (e != cudaSuccess) return e;
-    KTrace<NodeT, ANY, SPILL><<<grid, kTraceBlock, 0, stream>>>((const NodeT*)s->d_nodes, s->d_tris, d_rays, n,
-                                                                (int)s->tri_material.size(), hits, occ, chunk, counter,
-                                                                err);
+    KTrace<NodeT, ANY, SPILL, COOP><<<grid, kTraceBlock, 0, stream>>>((const NodeT*)s->d_nodes, s->d_tris, d_rays, n,
+                                                                      (int)s->tri_material.size(), hits, occ, chunk,
+                                                                      counter, err);
     return cudaGetLastError();
 }
 
-template <bool ANY>
-cudaError_t Dispatch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n, rtb200_hit* hits, uint8_t* occ,
-                     unsigned long long* counter, unsigned* err, cudaStream_t stream)
+template <class NodeT, bool ANY>
+cudaError_t Launch(const rtb200_scene* s, const rtb200_ray* d_rays, unsigned n, rtb200_hit* hits, uint8_t* occ,
+                   unsigned* counter, unsigned* err, cudaStream_t stream)
 {
-    if (n <= 0) return cudaSuccess;
     const bool spill = s->stack_bound > kTraceStack;
+    if (n <= kCoopBatchPerSm * (unsigned)s->ctx->num_sms)
+        return spill ? LaunchKernel<NodeT, ANY, true, true>(s, d_rays, n, hits, occ, counter, err, stream)
+                     : LaunchKernel<NodeT, ANY, false, true>(s, d_rays, n, hits, occ, counter, err, stream);
+    return spill ? LaunchKernel<NodeT, ANY, true, false>(s, d_rays, n, hits, occ, counter, err, stream)
+                 : LaunchKernel<NodeT, ANY, false, false>(s, d_rays, n, hits, occ, counter, err, stream);
+}
+
+template <bool ANY>
+cudaError_t DispatchPart(const rtb200_scene* s, const rtb200_ray* d_rays, unsigned n, rtb200_hit* hits, uint8_t* occ,
+                         unsigned* counter, unsigned* err, cudaStream_t stream)
+{
     if (s->layout == RTB200_BVH_W8) {
         static std::atomic<int> grids[kGridDevices];
-        int grid, chunk;
+        int grid;
+        unsigned chunk;
         const cudaError_t e = PlanFeed(KTraceW8<ANY>, grids, s->ctx, n, counter, stream, grid, chunk);
         if (e != cudaSuccess) return e;
         KTraceW8<ANY><<<grid, kTraceBlock, 0, stream>>>((const WNode8*)s->d_nodes, s->d_tris, d_rays, n, hits, occ,
                                                         chunk, counter, err);
         return cudaGetLastError();
     }
-    if (s->layout == RTB200_BVH_Q8)
-        return spill ? Launch<QNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream)
-                     : Launch<QNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
-    if (s->layout == RTB200_BVH_F16)
-        return spill ? Launch<HNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream)
-                     : Launch<HNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
-    return spill ? Launch<GpuNode4, ANY, true>(s, d_rays, n, hits, occ, counter, err, stream)
-                 : Launch<GpuNode4, ANY, false>(s, d_rays, n, hits, occ, counter, err, stream);
+    if (s->layout == RTB200_BVH_Q8) return Launch<QNode4, ANY>(s, d_rays, n, hits, occ, counter, err, stream);
+    if (s->layout == RTB200_BVH_F16) return Launch<HNode4, ANY>(s, d_rays, n, hits, occ, counter, err, stream);
+    return Launch<GpuNode4, ANY>(s, d_rays, n, hits, occ, counter, err, stream);
+}
+
+template <bool ANY>
+cudaError_t Dispatch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n, rtb200_hit* hits, uint8_t* occ,
+                     unsigned long long* counter, unsigned* err, cudaStream_t stream)
+{
+    cudaError_t e = cudaSuccess;
+    for (int64_t at = 0; at < n && e == cudaSuccess; at += kFeedRays)
+        e = DispatchPart<ANY>(s, d_rays + at, (unsigned)std::min<int64_t>(kFeedRays, n - at),
+                              ANY ? nullptr : hits + at, ANY ? occ + at : nullptr, (unsigned*)counter, err, stream);
+    return e;
 }
 
 }  // namespace
