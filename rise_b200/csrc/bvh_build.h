@@ -74,7 +74,8 @@ void MergeMeshBVHs(const std::vector<MeshBVH2>& meshes, BuiltBVH& out);
 
 // ---- device layouts -------------------------------------------------------
 
-// FP32 wide node: 4 child boxes as SoA float4 + child links, 128 bytes.
+// FP32 wide node: 4 child boxes as SoA float4, an axis' low and high planes side
+// by side (one 32-byte load), + child links, 128 bytes.
 // child[i] >= 0: internal node index; child[i] == INT32_MIN: empty slot;
 // other child[i] < 0: a leaf whose first triangle (in leaf order) is
 // ~child[i], holding count[i] triangles (the last one is flagged in
@@ -82,8 +83,9 @@ void MergeMeshBVHs(const std::vector<MeshBVH2>& meshes, BuiltBVH& out);
 // slots are known from the link); count[i] (-1 for an empty slot) is kept
 // for the host's view of the node.
 struct alignas(16) GpuNode4 {
-    float lox[4], loy[4], loz[4];
-    float hix[4], hiy[4], hiz[4];
+    float lox[4], hix[4];
+    float loy[4], hiy[4];
+    float loz[4], hiz[4];
     int32_t child[4];
     int32_t count[4];
 };
