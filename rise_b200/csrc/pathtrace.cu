@@ -324,9 +324,12 @@ KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int assign)
             const PtJobDev& J = jobs[jid];
             const unsigned long long g = a.base + (unsigned long long)(i - a.off);
             {   // PinholeCamera::GenerateRay (Cameras/PinholeCamera.cpp:182-210)
-                const uint32_t slot_px = (uint32_t)(g % (unsigned long long)J.npix);
+                // 64-bit division only where the request needs it.
+                const uint32_t npix = (uint32_t)J.npix;
+                const uint32_t pass = J.total >> 32 ? (uint32_t)(g / npix) : (uint32_t)g / npix;
+                const uint32_t slot_px = (uint32_t)g - pass * npix;
                 const uint32_t pixel = J.px_list ? __ldg(J.px_list + slot_px) : slot_px;
-                const uint32_t sample = (uint32_t)(J.sample_begin + g / (unsigned long long)J.npix);
+                const uint32_t sample = (uint32_t)(J.sample_begin + pass);
                 const int px = (int)(pixel % (uint32_t)J.cam.width), py = (int)(pixel / (uint32_t)J.cam.width);
                 const bool sobol = J.set.sampler != kSamplerHash, shuf = J.set.sampler == kSamplerSobolShuffled;
                 // Hash key, or the pixel's Sobol seed (camera dimensions 0-2).
@@ -614,7 +617,7 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
         float4 L = P.L[slot];
         const int depth = (int)(m.z & kFlagDepthMask);
         // Random numbers: hash key or Sobol seed in meta.w, sample index in meta.y.
-        VertexRng rng{m.w, m.y, depth, set.sampler, 0u};
+        VertexRng rng{m.w, m.y, depth, set.sampler, 0u, 0u, 0u};
         const float bsdfPdf = aux.y;
         unsigned term = (m.z >> kTermShift) & 0xfu;
         float lam[4];
@@ -860,6 +863,8 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
                 #pragma unroll 1
                 for (int k = 0; k < nsamp; ++k) {
                     if (set.nee_per_lambda && (term & (1u << k))) continue;
+                    // Wavelengths that share this light sample.
+                    const int j0 = set.nee_per_lambda ? k : 0, j1 = set.nee_per_lambda ? k + 1 : 4;
                     if (set.n_lights > 0) {
                         const float ul = rng.next(4 * k + 0);
                         int li = 0;
@@ -889,9 +894,8 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
                                 bool any = false;
                                 const GgxPair bq = NeePair(mtype, gp, ns, gnv, r, toL);
                                 #pragma unroll 1
-                                for (int j = 0; j < 4; ++j) {
+                                for (int j = j0; j < j1; ++j) {
                                     if (term & (1u << j)) continue;
-                                    if (set.nee_per_lambda && j != k) continue;
                                     const float f = NeeValue(mtype, M, ps, j, bq, gp.eavg, amb);
                                     const float v = Get(thr, j) * lg.le * f * cosS / (dist * dist) / psel;
                                     Set(c, j, v);
@@ -933,9 +937,8 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
                                 const GgxPair bq = NeePair(mtype, gp, ns, gnv, r, toL);
                                 const float pb = bq.pdf;
                                 #pragma unroll 1
-                                for (int j = 0; j < 4; ++j) {
+                                for (int j = j0; j < j1; ++j) {
                                     if (term & (1u << j)) continue;
-                                    if (set.nee_per_lambda && j != k) continue;
                                     const float f = NeeValue(mtype, M, ps, j, bq, gp.eavg, amb);
                                     const float w = (pb > 0.0f ? PowerHeuristic(plight, pb) : 1.0f) / psel;
                                     const float v = Get(thr, j) * Spec(S.spectra, lg.emit, lam[j]) * cosS * geom * f * w;
@@ -979,9 +982,8 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
                             const GgxPair bq = NeePair(mtype, gp, ns, gnv, r, dir);
                             const float pb = bq.pdf;
                             #pragma unroll 1
-                            for (int j = 0; j < 4; ++j) {
+                            for (int j = j0; j < j1; ++j) {
                                 if (term & (1u << j)) continue;
-                                if (set.nee_per_lambda && j != k) continue;
                                 const float f = NeeValue(mtype, M, ps, j, bq, gp.eavg, amb);
                                 const float w = pb > 0.0f ? PowerHeuristic(epdf, pb) : 1.0f;
                                 const float le = (ENV && S.env_map) ? EnvSpectrum(es, lam[j])

@@ -14,9 +14,26 @@ constexpr float kPi = 3.14159265358979323846f;
 constexpr float kInvPi = 0.31830988618379067154f;
 constexpr float kNearZero = 1e-12f;   // NEARZERO, Utilities/Math3D/Constants.h:33
 
-// Defined here: this header is compiled into exactly one translation unit
-// (pathtrace.cu).
-__constant__ float c_cie[3][RTB200_CIE_COUNT] = {{RTB200_CIE_XBAR}, {RTB200_CIE_YBAR}, {RTB200_CIE_ZBAR}};
+// The colour-matching functions, a row (x, y, z, 0) per wavelength, in global
+// memory: every lane of a warp reads its own wavelength, which constant memory
+// would serialise (24 scalar reads a sample; KRegen spent most of its time
+// there).  Defined here: this header is compiled into exactly one translation
+// unit (pathtrace.cu).
+struct alignas(16) CieTable {
+    float v[RTB200_CIE_COUNT][4];
+};
+constexpr CieTable MakeCieTable()
+{
+    constexpr float x[] = {RTB200_CIE_XBAR}, y[] = {RTB200_CIE_YBAR}, z[] = {RTB200_CIE_ZBAR};
+    CieTable t{};
+    for (int i = 0; i < RTB200_CIE_COUNT; ++i) {
+        t.v[i][0] = x[i];
+        t.v[i][1] = y[i];
+        t.v[i][2] = z[i];
+    }
+    return t;
+}
+__device__ const CieTable g_cie = MakeCieTable();
 
 // ---- random numbers ---------------------------------------------------------
 // Counter-based: every number is a hash of (seed, pixel, sample, dimension),
@@ -64,21 +81,25 @@ __device__ __forceinline__ uint32_t HashCombine(uint32_t a, uint32_t b)
     return a;
 }
 
-__device__ __forceinline__ uint32_t SobolDim1(uint32_t i)
+// Sobol dimension 1 of i, bit-reversed.  Over GF(2) the direction numbers are
+// the powers of (1 + x) applied to 1 (bit 31 - k holding x^k), so the XOR over
+// the set bits of i is the polynomial i shifted by one, i(1 + x); splitting i
+// into halves, (1 + x)^(2^k) = 1 + x^(2^k) adds the upper half to the lower, at
+// every size.  Ten instructions where the sum over the bits of a shuffled
+// index, which has all 32, took a loop of 32 steps.
+__device__ __forceinline__ uint32_t SobolDim1Reversed(uint32_t i)
 {
-    uint32_t v = 0, d = 1u << 31;
-    while (i) {
-        if (i & 1u) v ^= d;
-        d ^= d >> 1;
-        i >>= 1;
-    }
-    return v;
+    i ^= i >> 16;
+    i ^= (i >> 8) & 0x00ff00ffu;
+    i ^= (i >> 4) & 0x0f0f0f0fu;
+    i ^= (i >> 2) & 0x33333333u;
+    i ^= (i >> 1) & 0x55555555u;
+    return i;
 }
 
-// Owen scrambling by the Laine-Karras hash on the bit-reversed value.
-__device__ __forceinline__ uint32_t OwenScramble(uint32_t v, uint32_t s)
+// Owen scrambling by the Laine-Karras hash on the bit-reversed value v.
+__device__ __forceinline__ uint32_t OwenScrambleReversed(uint32_t v, uint32_t s)
 {
-    v = __brev(v);
     v ^= v * 0x3d20adeau;
     v += s;
     v *= (s >> 16) | 1u;
@@ -92,11 +113,21 @@ __device__ __forceinline__ uint32_t OwenScramble(uint32_t v, uint32_t s)
 // ("Practical Hash-based Owen Scrambling", JCGT 9(4), 2020, section 4), so
 // different pairs no longer replay one Sobol pair under another scramble;
 // the reference pads without it.
-__device__ __forceinline__ float SobolSample(uint32_t index, uint32_t dim, uint32_t seed, bool shuffle = false)
+__device__ __forceinline__ uint32_t SobolShuffle(uint32_t index, uint32_t pair, uint32_t seed)
 {
-    if (shuffle) index = OwenScramble(index, HashCombine(HashCombine(seed, 0x5bd1e995u), dim >> 1));
-    const uint32_t v = OwenScramble((dim & 1u) ? SobolDim1(index) : __brev(index), HashCombine(seed, dim));
+    return OwenScrambleReversed(__brev(index), HashCombine(HashCombine(seed, 0x5bd1e995u), pair));
+}
+
+// Dimension `dim` of the (shuffled) index.
+__device__ __forceinline__ float SobolValue(uint32_t index, uint32_t dim, uint32_t seed)
+{
+    const uint32_t v = OwenScrambleReversed((dim & 1u) ? SobolDim1Reversed(index) : index, HashCombine(seed, dim));
     return (float)(v >> 8) * (1.0f / 16777216.0f);   // the top 24 bits: < 1 in FP32
+}
+
+__device__ __forceinline__ float SobolSample(uint32_t index, uint32_t dim, uint32_t seed, bool shuffle)
+{
+    return SobolValue(shuffle ? SobolShuffle(index, dim >> 1, seed) : index, dim, seed);
 }
 
 // Sobol seed of a pixel: the reference's HashCombine(x, y); a nonzero job seed
@@ -119,11 +150,19 @@ struct VertexRng {
     int depth;
     int mode;          // kSamplerHash / kSamplerSobol / kSamplerSobolShuffled
     uint32_t cur;
+    // The last dimension pair drawn from (dimensions start at 512) and its
+    // shuffled index: a pair's two numbers come one after the other.
+    uint32_t pair, shuffled;
     __device__ __forceinline__ float next(int j)
     {
-        if (mode != kSamplerHash)
-            return SobolSample(index, (16u + (uint32_t)depth) * 32u + cur++, key, mode == kSamplerSobolShuffled);
-        return Rand(key, Dim(depth, j));
+        if (mode == kSamplerHash) return Rand(key, Dim(depth, j));
+        const uint32_t dim = (16u + (uint32_t)depth) * 32u + cur++;
+        if (mode == kSamplerSobol) return SobolValue(index, dim, key);
+        if ((dim >> 1) != pair) {
+            pair = dim >> 1;
+            shuffled = SobolShuffle(index, pair, key);
+        }
+        return SobolValue(shuffled, dim, key);
     }
     __device__ __forceinline__ void skip(int n) { cur += (uint32_t)n; }
 };
@@ -183,21 +222,28 @@ __device__ __forceinline__ bool Cmf(float nm, float& X, float& Y, float& Z)
     const int i = (int)floorf(x);
     const int j = i + 1 > 80 ? 80 : i + 1;
     const float w = x - (float)i;
-    X = c_cie[0][i] + w * (c_cie[0][j] - c_cie[0][i]);
-    Y = c_cie[1][i] + w * (c_cie[1][j] - c_cie[1][i]);
-    Z = c_cie[2][i] + w * (c_cie[2][j] - c_cie[2][i]);
+    const float4 a = __ldg(reinterpret_cast<const float4*>(g_cie.v[i]));
+    const float4 b = __ldg(reinterpret_cast<const float4*>(g_cie.v[j]));
+    X = a.x + w * (b.x - a.x);
+    Y = a.y + w * (b.y - a.y);
+    Z = a.z + w * (b.z - a.z);
     return true;
 }
 
 // SampledWavelengths::SampleEquidistant
-// (src/Library/Utilities/Color/SampledWavelengths.h:79-106).
+// (src/Library/Utilities/Color/SampledWavelengths.h:79-106).  The offset from
+// lmin lies in [0, 1.75 range], where fmod by the range is at most one exact
+// subtraction.
 __device__ __forceinline__ void Wavelengths(float hero, float lmin, float lmax, float lam[4])
 {
     const float range = lmax - lmin;
     const float delta = range * 0.25f;
     lam[0] = hero;
 #pragma unroll
-    for (int i = 1; i < 4; ++i) lam[i] = lmin + fmodf(hero - lmin + (float)i * delta, range);
+    for (int i = 1; i < 4; ++i) {
+        const float x = hero - lmin + (float)i * delta;
+        lam[i] = lmin + (x >= range ? x - range : x);
+    }
 }
 
 __device__ __forceinline__ float Get(const float4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
