@@ -314,19 +314,34 @@ __device__ __forceinline__ float PowerHeuristic(float a, float b)
     return a2 / (a2 + b * b);
 }
 
-// Warp-aggregated queue append: one atomic per warp; returns this lane's
-// index (or -1 when `pred` is false).
-__device__ __forceinline__ int WarpAppend(int* counter, bool pred)
+// Appends to up to three queues at once, called by a whole warp: a lane adds
+// n[q] entries to queue q and gets its first index in at[q].  The counts
+// (below 1024 a warp) are summed in one packed scan and the counters advanced
+// by one instruction, an atomic per queue and warp.
+template <int N>
+__device__ __forceinline__ void WarpAppend(int* const (&counter)[N], const int (&n)[N], int (&at)[N])
 {
-    const unsigned act = __activemask();
-    const unsigned m = __ballot_sync(act, pred);
-    if (!m) return -1;
+    static_assert(N <= 3, "three packed counts");
     const int lane = threadIdx.x & 31;
-    const int leader = __ffs(m) - 1;
+    unsigned mine = 0;
+#pragma unroll
+    for (int q = 0; q < N; ++q) mine |= (unsigned)n[q] << (10 * q);
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
     int base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(m));
-    base = __shfl_sync(act, base, leader);
-    return pred ? base + __popc(m & ((1u << lane) - 1u)) : -1;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        const int t = (int)((total >> (10 * q)) & 1023u);
+        if (lane == q && t) base = atomicAdd(counter[q], t);
+    }
+    const unsigned excl = incl - mine;
+#pragma unroll
+    for (int q = 0; q < N; ++q) at[q] = __shfl_sync(0xffffffffu, base, q) + (int)((excl >> (10 * q)) & 1023u);
 }
 
 }  // namespace rtb200
