@@ -118,7 +118,7 @@ struct rtb200_engine {
     unsigned long long* d_ctr = nullptr;   // [kMaxJobs] issued, [kMaxJobs] done
     PtJobDev* h_table = nullptr;           // pinned
     int* h_ids = nullptr;                  // pinned
-    int* h_cnt = nullptr;                  // pinned
+    int* h_cnt = nullptr;                  // pinned: counters, then the error word
     unsigned long long* h_ctr = nullptr;   // pinned
     rtb200_job* owner[kMaxJobs] = {};
     unsigned long long total[kMaxJobs] = {};
@@ -167,6 +167,12 @@ PtLaunch MakeLaunch(const rtb200_engine* e)
     L.paths = e->paths;
     L.queues = e->queues;
     L.sms = e->ctx->num_sms;
+    // Idle here: the casts that use these streams finish under the same lock.
+    L.side[0] = e->ctx->trace2;
+    L.side[1] = e->ctx->copy_in;
+    L.fork = e->ctx->ev_up[0];
+    L.join[0] = e->ctx->ev_trace[0];
+    L.join[1] = e->ctx->ev_down[0];
     return L;
 }
 
@@ -219,7 +225,7 @@ int EngineCreate(rtb200_ctx* ctx, int capacity, rtb200_engine** out)
     }
     if (cudaMallocHost(&e->h_table, sizeof(PtJobDev) * kMaxJobs) != cudaSuccess ||
         cudaMallocHost(&e->h_ids, 4 * (kMaxJobs + 1)) != cudaSuccess ||
-        cudaMallocHost(&e->h_cnt, 4 * kCntCount) != cudaSuccess ||
+        cudaMallocHost(&e->h_cnt, 4 * (kCntCount + 1)) != cudaSuccess ||
         cudaMallocHost(&e->h_ctr, 8 * 2 * kMaxJobs) != cudaSuccess || cudaEventCreate(&e->e0) != cudaSuccess ||
         cudaEventCreate(&e->e1) != cudaSuccess) {
         cudaGetLastError();
@@ -318,7 +324,7 @@ int EngineStep(rtb200_engine* e, int iterations, bool graph)
         // Every slot starts free; statistics counters restart from zero.
         cudaMemcpyAsync(e->queues.free_, e->d_iota, 4 * (size_t)e->capacity, cudaMemcpyDeviceToDevice, st);
         int init[kCntCount] = {0};
-        init[kCntFree] = e->capacity;
+        init[kCntFreeNext] = e->capacity;   // the first iteration rotates it into place
         std::memcpy(e->h_cnt, init, sizeof(init));
         cudaMemcpyAsync(e->queues.cnt, e->h_cnt, 4 * kCntCount, cudaMemcpyHostToDevice, st);
         e->fresh = false;
@@ -386,14 +392,16 @@ int EngineStep(rtb200_engine* e, int iterations, bool graph)
     }
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(e->h_cnt, e->queues.cnt, 4 * kCntCount, cudaMemcpyDeviceToHost, st);
+    if (err == cudaSuccess)
+        err = cudaMemcpyAsync(e->h_cnt + kCntCount, e->queues.err, 4, cudaMemcpyDeviceToHost, st);
     if (err == cudaSuccess) err = cudaMemcpyAsync(e->h_ctr, e->d_ctr, 8 * 2 * kMaxJobs, cudaMemcpyDeviceToHost, st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(st);
     if (err != cudaSuccess) return CudaCheck(ctx, err, "wavefront step");
-    unsigned errw = 0;
-    cudaMemcpy(&errw, e->queues.err, 4, cudaMemcpyDeviceToHost);
-    if (errw) return SetError(ctx, RTB200_E_DEVICE, "device error word set (traversal stack overflow)");
-    // Per-job statistics: attribute this step's segments to the active jobs.
-    const long long seg = (unsigned)e->h_cnt[kCntSegments], sh = (unsigned)e->h_cnt[kCntShadowRays];
+    if (e->h_cnt[kCntCount]) return SetError(ctx, RTB200_E_DEVICE, "device error word set (traversal stack overflow)");
+    // Per-job statistics: attribute this step's segments to the active jobs
+    // (the last iteration's are still in its queue counters).
+    const long long seg = (unsigned)e->h_cnt[kCntSegments] + (unsigned)e->h_cnt[kCntActive],
+                    sh = (unsigned)e->h_cnt[kCntShadowRays] + (unsigned)e->h_cnt[kCntShadow];
     const long long dseg = seg - e->seg_seen, dsh = sh - e->shadow_seen;
     e->seg_seen = seg;
     e->shadow_seen = sh;

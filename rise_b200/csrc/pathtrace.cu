@@ -6,9 +6,10 @@
 // PathTracingSpectralRasterizer::IntegratePixelSpectral
 // (src/Library/Rendering/PathTracingSpectralRasterizer.cpp:121-198).
 //
-// A fixed pool of path slots lives in HBM as SoA.  One iteration is seven
+// A fixed pool of path slots lives in HBM as SoA.  One iteration is six
 // launches over device-side queues (no host round trip):
-//   KAssign  split the free slots among the jobs that have samples left
+//   KAssign  rotate the queue counters, split the free slots among the jobs
+//            that have samples left
 //   KRegen   splat finished paths into the film, start new camera samples
 //   KExtend  closest hit for every active path (warp while-while traversal)
 //   KClassify sort the active paths by the material they hit
@@ -17,7 +18,6 @@
 //            companion-wavelength weights, Russian roulette
 //   KConnect any hit for the shadow-ray queue; unoccluded contributions are
 //            added to the path's per-wavelength radiance
-//   KSwap    rotate queue counters
 // Appends to queues are warp-aggregated (one atomic per warp).
 #include <cfloat>
 
@@ -195,14 +195,16 @@ __device__ __forceinline__ void Splat(const PtPaths& P, const PtJobDev& J, int s
 
 // ---- kernels ---------------------------------------------------------------
 
-// Inclusive prefix sum over a block of up to 1024 threads.
-__device__ __forceinline__ int BlockScan(int v, int* warp_sums)
+// Inclusive prefix sum over a block of 1024 threads, or over one warp.
+template <bool WARP>
+__device__ __forceinline__ int Scan(int v, int* warp_sums)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int o = 1; o < 32; o <<= 1) {
         const int u = __shfl_up_sync(kFull, v, o);
         if (lane >= o) v += u;
     }
+    if (WARP) return v;
     if (lane == 31) warp_sums[w] = v;
     __syncthreads();
     if (w == 0) {
@@ -229,16 +231,16 @@ __device__ __forceinline__ int BlockScan(int v, int* warp_sums)
 // share.  Block prefix sums replace per-warp atomics on one counter per job.
 // Images do not depend on this schedule: a sample's random numbers depend
 // only on its job, pixel and sample index.
-__global__ void __launch_bounds__(kPtMaxJobs)
-KAssign(const PtJobDev* __restrict__ jobs, const int* __restrict__ ids, PtQueues Q, int iter)
+template <bool WARP>
+__device__ __forceinline__ void AssignJobs(const PtJobDev* __restrict__ jobs, const int* __restrict__ ids,
+                                           const PtQueues& Q, int iter, int njobs, int n)
 {
-    const int njobs = Q.cnt[kCntJobs];
     __shared__ int sums[32];
     __shared__ unsigned long long s_left[kPtMaxJobs];   // samples left per job (for the order)
     __shared__ int s_sorted[kPtMaxJobs];
     __shared__ int s_live, s_first;
-    const int t = threadIdx.x;
-    const int n = Q.cnt[kCntFree];
+    const auto sync = [] { if (WARP) __syncwarp(); else __syncthreads(); };
+    const int t = threadIdx.x, last = WARP ? 31 : kPtMaxJobs - 1;
     int jid = -1, rem = 0;
     unsigned long long issued = 0, left_all = 0;
     if (t < njobs) {
@@ -250,15 +252,15 @@ KAssign(const PtJobDev* __restrict__ jobs, const int* __restrict__ ids, PtQueues
             rem = (int)min(left_all, (unsigned long long)n);
         }
     }
-    const int live = BlockScan(rem > 0 ? 1 : 0, sums);
-    if (t == blockDim.x - 1) s_live = live;
-    __syncthreads();
+    const int live = Scan<WARP>(rem > 0 ? 1 : 0, sums);
+    if (t == last) s_live = live;
+    sync();
     const int share = s_live > 0 ? n / s_live / 4 : 0;
     const int first = min(rem, share);
-    const int firstIncl = BlockScan(first, sums);
-    if (t == blockDim.x - 1) s_first = firstIncl;
+    const int firstIncl = Scan<WARP>(first, sums);
+    if (t == last) s_first = firstIncl;
     s_left[t] = left_all;
-    __syncthreads();
+    sync();
     const int left = n - s_first;
     const int more = rem - first;
     // Rank by samples left (ties by position), then a prefix sum in that order.
@@ -266,14 +268,15 @@ KAssign(const PtJobDev* __restrict__ jobs, const int* __restrict__ ids, PtQueues
     if (t < njobs)
         for (int k = 0; k < njobs; ++k) rank += (s_left[k] < left_all) || (s_left[k] == left_all && k < t);
     if (t < njobs) s_sorted[rank] = more;
-    __syncthreads();
+    sync();
     const int v = t < njobs ? s_sorted[t] : 0;
-    const int inclSorted = BlockScan(v, sums);
+    const int inclSorted = Scan<WARP>(v, sums);
+    sync();
     s_sorted[t] = inclSorted - v;   // exclusive prefix in rank order
-    __syncthreads();
+    sync();
     const int extra = t < njobs ? max(0, min(more, left - s_sorted[rank])) : 0;
     const int take = first + extra;
-    const int takeIncl = BlockScan(take, sums);
+    const int takeIncl = Scan<WARP>(take, sums);
     if (t < njobs) {
         PtAssign a;
         a.base = issued;
@@ -282,15 +285,39 @@ KAssign(const PtJobDev* __restrict__ jobs, const int* __restrict__ ids, PtQueues
         Q.assign[t] = a;
         if (take > 0) *jobs[jid].sample_ctr = issued + (unsigned long long)take;
     }
-    if (t == blockDim.x - 1) Q.cnt[kCntAssigned] = takeIncl;
+    if (t == last) Q.cnt[kCntAssigned] = takeIncl;
+}
+
+// Also rotates the queue counters of the last iteration into this one's: a
+// launch of its own for that, and a memset of the feed counters, cost 4 us an
+// iteration.  With up to 32 jobs one warp does the work.
+__global__ void __launch_bounds__(kPtMaxJobs)
+KAssign(const PtJobDev* __restrict__ jobs, const int* __restrict__ ids, PtQueues Q, int iter)
+{
+    const int njobs = Q.cnt[kCntJobs], n = Q.cnt[kCntFreeNext];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int* cnt = Q.cnt;
+        for (int c = 0; c < kShadeClasses; ++c) cnt[kCntClass + c] = 0;
+        cnt[kCntSegments] += cnt[kCntActive];
+        cnt[kCntShadowRays] += cnt[kCntShadow];
+        cnt[kCntActive] = cnt[kCntActiveNext];
+        cnt[kCntActiveNext] = 0;
+        cnt[kCntFree] = n;
+        cnt[kCntFreeNext] = 0;
+        cnt[kCntShadow] = 0;
+        Q.trace_ctr[0] = Q.trace_ctr[1] = 0ull;
+    }
+    if (njobs > 32) AssignJobs<false>(jobs, ids, Q, iter, njobs, n);
+    else if (threadIdx.x < 32) AssignJobs<true>(jobs, ids, Q, iter, njobs, n);
 }
 
 __global__ void __launch_bounds__(kShadeBlock)
-KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int assign)
+KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
 {
     const int njobs = Q.cnt[kCntJobs];
     const int n = Q.cnt[kCntFree];
-    const int nassigned = assign ? Q.cnt[kCntAssigned] : 0;
+    const int nassigned = Q.cnt[kCntAssigned];
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1168,18 +1195,6 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
     }
 }
 
-__global__ void KSwap(int* cnt)
-{
-    for (int c = 0; c < kShadeClasses; ++c) cnt[kCntClass + c] = 0;
-    cnt[kCntSegments] += cnt[kCntActive];
-    cnt[kCntShadowRays] += cnt[kCntShadow];
-    cnt[kCntActive] = cnt[kCntActiveNext];
-    cnt[kCntActiveNext] = 0;
-    cnt[kCntFree] = cnt[kCntFreeNext];
-    cnt[kCntFreeNext] = 0;
-    cnt[kCntShadow] = 0;
-}
-
 // Kahan-compensated fold of this call's film into the running sums.
 __global__ void KFold(float* pass, float* sum, float* comp, int n)
 {
@@ -1342,17 +1357,25 @@ cudaError_t PtIteration(const PtLaunch& L, int iter, cudaStream_t st)
 {
     const int shadeGrid = L.sms * 8;
     KAssign<<<1, kPtMaxJobs, 0, st>>>(L.jobs, L.ids, L.queues, iter);
-    KRegen<<<shadeGrid, kShadeBlock, 0, st>>>(L.jobs, L.paths, L.queues, 1);
-    cudaMemsetAsync(L.queues.trace_ctr, 0, 2 * sizeof(unsigned long long), st);
+    KRegen<<<shadeGrid, kShadeBlock, 0, st>>>(L.jobs, L.paths, L.queues);
     if (L.layout == RTB200_BVH_Q8) LaunchTrace<QNode4>(L, st, true);
     else if (L.layout == RTB200_BVH_F16) LaunchTrace<HNode4>(L, st, true);
     else LaunchTrace<GpuNode4>(L, st, true);
     if (L.classify) {
         KClassify<<<shadeGrid, kShadeBlock, 0, st>>>(L.jobs, L.paths, L.queues);
-        LaunchShade<0>(L, 1, st);
+        // The classes side by side: a late iteration's few paths are a wait for
+        // one warp's instructions in each (9,600 pixels at 4 spp: 57, 27 and 9 us).
+        cudaEventRecord(L.fork, st);
+        cudaStreamWaitEvent(L.side[0], L.fork, 0);
+        cudaStreamWaitEvent(L.side[1], L.fork, 0);
         LaunchShade<1>(L, 1, st);
+        LaunchShade<0>(L, 1, L.side[0]);
         // Dielectrics shade neither escaped rays nor next events.
-        KShade<2, false><<<shadeGrid, kShadeBlock, 0, st>>>(L.jobs, L.paths, L.queues, 1);
+        KShade<2, false><<<shadeGrid, kShadeBlock, 0, L.side[1]>>>(L.jobs, L.paths, L.queues, 1);
+        for (int k = 0; k < 2; ++k) {
+            cudaEventRecord(L.join[k], L.side[k]);
+            cudaStreamWaitEvent(st, L.join[k], 0);
+        }
     } else if (L.shade_class == 0) {
         LaunchShade<0>(L, 0, st);
     } else if (L.shade_class == 1) {
@@ -1366,13 +1389,6 @@ cudaError_t PtIteration(const PtLaunch& L, int iter, cudaStream_t st)
     if (L.layout == RTB200_BVH_Q8) LaunchTrace<QNode4>(L, st, false);
     else if (L.layout == RTB200_BVH_F16) LaunchTrace<HNode4>(L, st, false);
     else LaunchTrace<GpuNode4>(L, st, false);
-    KSwap<<<1, 1, 0, st>>>(L.queues.cnt);
-    return cudaGetLastError();
-}
-
-cudaError_t PtDrain(const PtLaunch& L, cudaStream_t st)
-{
-    KRegen<<<L.sms * 8, kShadeBlock, 0, st>>>(L.jobs, L.paths, L.queues, 0);
     return cudaGetLastError();
 }
 

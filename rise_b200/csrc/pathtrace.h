@@ -24,14 +24,15 @@ struct PtLaunch {
     PtPaths paths;
     PtQueues queues;
     int sms;
+    // Streams and events the shading classes run side by side with.
+    cudaStream_t side[2];
+    cudaEvent_t fork, join[2];
 };
 
-// One wavefront iteration (regenerate, extend, shade, connect, swap counters),
+// One wavefront iteration (rotate counters, regenerate, extend, shade, connect),
 // asynchronous on `st`.  The caller swaps queues.active/active_next and
 // queues.free_/free_next after each call.
 cudaError_t PtIteration(const PtLaunch& L, int iter, cudaStream_t st);
-// Splat paths still marked finished into their films (end of a render).
-cudaError_t PtDrain(const PtLaunch& L, cudaStream_t st);
 // Upload the GGX E_ss (32 x 32), E_avg (32), multiple-scattering lobe
 // normalisation (32) and cumulative segment integral (32 x 34) tables.
 cudaError_t PtSetGgxTables(const float* ess, const float* eavg, const float* msz, const float* mscum,
