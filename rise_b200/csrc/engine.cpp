@@ -713,35 +713,17 @@ int rtb200_job_read_film(rtb200_job* j, float* xyz)
     std::lock_guard<std::mutex> g(ctx->mu);
     if (j->engine) return SetError(ctx, RTB200_E_NOT_READY, "job has a request in flight");
     cudaSetDevice(ctx->device);
-    const size_t n = (size_t)j->film_n;
-    std::vector<double> acc(n);
-    if (j->wide) {
-        const cudaError_t e = cudaMemcpy(acc.data(), j->wide, 8 * n, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return CudaCheck(ctx, e, "film readback");
-    } else {
-        std::vector<float> sum(n), comp(n);
-        cudaError_t e = cudaMemcpy(sum.data(), j->sum, 4 * n, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(comp.data(), j->comp, 4 * n, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return CudaCheck(ctx, e, "film readback");
-        for (size_t i = 0; i < n; ++i) acc[i] = (double)sum[i] - (double)comp[i];
-    }
-    if (j->channels == 3 && j->adaptive) {
-        std::vector<unsigned> cnt((size_t)j->npix);
-        const cudaError_t e = cudaMemcpy(cnt.data(), j->counts, 4 * cnt.size(), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return CudaCheck(ctx, e, "film readback");
-        for (size_t i = 0; i < n; ++i) xyz[i] = cnt[i / 3] ? (float)(acc[i] / (double)cnt[i / 3]) : 0.0f;
-    } else if (j->channels == 3) {
-        const double inv = j->spp_done > 0 ? 1.0 / (double)j->spp_done : 0.0;
-        for (size_t i = 0; i < n; ++i) xyz[i] = (float)(acc[i] * inv);
-    } else {
-        // FilteredFilm resolve (Rendering/FilteredFilm.cpp:100-132): weighted
-        // sum over the weight; pixels no sample reached stay 0.
-        for (size_t p = 0; p < (size_t)j->npix; ++p) {
-            const double w = acc[4 * p + 3];
-            for (int c = 0; c < 3; ++c) xyz[3 * p + c] = std::fabs(w) > 1e-10 ? (float)(acc[4 * p + c] / w) : 0.0f;
-        }
-    }
-    return RTB200_OK;
+    // Resolved on the device into the request accumulator, which is clear
+    // between requests and cleared again, so reading needs no memory.
+    const double inv = j->spp_done > 0 ? 1.0 / (double)j->spp_done : 0.0;
+    cudaError_t e = PtResolveFilm(j->sum, j->comp, j->wide, j->adaptive ? j->counts : nullptr, j->channels, inv, j->npix,
+                                  j->pass, ctx->num_sms, ctx->stream);
+    const size_t bytes = 12 * (size_t)j->npix;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(xyz, j->pass, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    const cudaError_t ec = cudaMemsetAsync(j->pass, 0, bytes, ctx->stream);
+    if (e == cudaSuccess) e = ec;
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    return CudaCheck(ctx, e, "film readback");
 }
 
 int rtb200_job_relmse(rtb200_job* j, const float* ref_xyz, double* relmse)

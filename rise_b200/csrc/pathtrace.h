@@ -49,6 +49,10 @@ cudaError_t PtFoldWide(float* pass, float* sum, float* comp, double* wide, int n
 // accumulation.
 cudaError_t PtRelMse(const float* sum, const float* comp, const double* wide, const unsigned* counts,
                      const float* ref, int npix, int channels, double inv_spp, double* out, int sms, cudaStream_t st);
+// out[3 p + k] = the resolved film in FP32 (resolve.cu): the mean of a pixel's
+// XYZ (sum * inv_spp, or sum / counts[p]) or weighted sum / weight.
+cudaError_t PtResolveFilm(const float* sum, const float* comp, const double* wide, const unsigned* counts,
+                          int channels, double inv_spp, int npix, float* out, int sms, cudaStream_t st);
 // Resolve the film to colour (resolve.cu): linear Rec.709 into rgb (3 floats
 // per pixel) when rgb is given, else 8-bit sRGB after exposure (ev_mul) and
 // the RTB200_TONE_* curve into rgb8.
