@@ -73,10 +73,11 @@ int DevAllocCached(rtb200_ctx* ctx, void** p, size_t bytes)
 void DevFreeCached(rtb200_ctx* ctx, void* p, size_t bytes)
 {
     if (!p) return;
-    if (ctx->cached + bytes > kDevCacheBytes) {
+    if (bytes > kDevCacheBytes) {
         DevFree(ctx, p, bytes);
         return;
     }
+    if (ctx->cached + bytes > kDevCacheBytes) DevReleaseCache(ctx);
     ctx->cache[bytes].push_back(p);
     ctx->cached += bytes;
     ctx->in_use -= bytes;
@@ -229,6 +230,7 @@ int rtb200_ctx_destroy(rtb200_ctx* ctx)
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     DevReleaseCache(ctx);
+    for (void* p : ctx->pinned) cudaFreeHost(p);
     for (int b = 0; b < 2; ++b) {
         cudaEventDestroy(ctx->ev_up[b]);
         cudaEventDestroy(ctx->ev_trace[b]);

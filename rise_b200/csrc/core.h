@@ -29,6 +29,8 @@ struct rtb200_ctx {
     // synchronise the device each time).  Not counted in in_use.
     std::unordered_map<size_t, std::vector<void*>> cache;
     size_t cached = 0;
+    // Pinned blocks of destroyed engines, all of one size (engine.cpp).
+    std::vector<void*> pinned;
 };
 
 struct rtb200_scene {
@@ -136,7 +138,9 @@ int DevAlloc(rtb200_ctx* ctx, void** p, size_t bytes);
 void DevFree(rtb200_ctx* ctx, void* p, size_t bytes);
 // The same for blocks used only by work on ctx->stream: a freed block is kept
 // (up to kDevCacheBytes in all) and handed to the next request of the same
-// size, which stream order makes safe.  DevReleaseCache returns them all.
+// size, which stream order makes safe.  DevReleaseCache returns them all; a
+// full cache is returned before the next block is kept, so sizes no longer
+// asked for do not crowd out those that are.
 constexpr size_t kDevCacheBytes = size_t(4) << 30;
 int DevAllocCached(rtb200_ctx* ctx, void** p, size_t bytes);
 void DevFreeCached(rtb200_ctx* ctx, void* p, size_t bytes);

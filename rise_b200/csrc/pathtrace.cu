@@ -1195,6 +1195,11 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
     }
 }
 
+__global__ void KIota(int* p, int n)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = i;
+}
+
 // Kahan-compensated fold of this call's film into the running sums.
 __global__ void KFold(float* pass, float* sum, float* comp, int n)
 {
@@ -1389,6 +1394,12 @@ cudaError_t PtIteration(const PtLaunch& L, int iter, cudaStream_t st)
     if (L.layout == RTB200_BVH_Q8) LaunchTrace<QNode4>(L, st, false);
     else if (L.layout == RTB200_BVH_F16) LaunchTrace<HNode4>(L, st, false);
     else LaunchTrace<GpuNode4>(L, st, false);
+    return cudaGetLastError();
+}
+
+cudaError_t PtIota(int* p, int n, int sms, cudaStream_t st)
+{
+    KIota<<<sms * 4, 256, 0, st>>>(p, n);
     return cudaGetLastError();
 }
 

@@ -53,6 +53,8 @@ cudaError_t PtRelMse(const float* sum, const float* comp, const double* wide, co
 // XYZ (sum * inv_spp, or sum / counts[p]) or weighted sum / weight.
 cudaError_t PtResolveFilm(const float* sum, const float* comp, const double* wide, const unsigned* counts,
                           int channels, double inv_spp, int npix, float* out, int sms, cudaStream_t st);
+// p[i] = i for the first n entries.
+cudaError_t PtIota(int* p, int n, int sms, cudaStream_t st);
 // Resolve the film to colour (resolve.cu): linear Rec.709 into rgb (3 floats
 // per pixel) when rgb is given, else 8-bit sRGB after exposure (ev_mul) and
 // the RTB200_TONE_* curve into rgb8.
