@@ -314,18 +314,20 @@ __device__ __forceinline__ float PowerHeuristic(float a, float b)
     return a2 / (a2 + b * b);
 }
 
-// Appends to up to three queues at once, called by a whole warp: a lane adds
+// Appends to up to four queues at once, called by a whole warp: a lane adds
 // n[q] entries to queue q and gets its first index in at[q].  The counts
-// (below 1024 a warp) are summed in one packed scan and the counters advanced
-// by one instruction, an atomic per queue and warp.
+// (below 1024 a warp, 256 with four queues) are summed in one packed scan and
+// the counters advanced by one instruction, an atomic per queue and warp.
 template <int N>
 __device__ __forceinline__ void WarpAppend(int* const (&counter)[N], const int (&n)[N], int (&at)[N])
 {
-    static_assert(N <= 3, "three packed counts");
+    static_assert(N <= 4, "packed counts");
+    constexpr int kBits = N <= 3 ? 10 : 8;
+    constexpr unsigned kMask = (1u << kBits) - 1u;
     const int lane = threadIdx.x & 31;
     unsigned mine = 0;
 #pragma unroll
-    for (int q = 0; q < N; ++q) mine |= (unsigned)n[q] << (10 * q);
+    for (int q = 0; q < N; ++q) mine |= (unsigned)n[q] << (kBits * q);
     unsigned incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -336,12 +338,12 @@ __device__ __forceinline__ void WarpAppend(int* const (&counter)[N], const int (
     int base = 0;
 #pragma unroll
     for (int q = 0; q < N; ++q) {
-        const int t = (int)((total >> (10 * q)) & 1023u);
+        const int t = (int)((total >> (kBits * q)) & kMask);
         if (lane == q && t) base = atomicAdd(counter[q], t);
     }
     const unsigned excl = incl - mine;
 #pragma unroll
-    for (int q = 0; q < N; ++q) at[q] = __shfl_sync(0xffffffffu, base, q) + (int)((excl >> (10 * q)) & 1023u);
+    for (int q = 0; q < N; ++q) at[q] = __shfl_sync(0xffffffffu, base, q) + (int)((excl >> (kBits * q)) & kMask);
 }
 
 }  // namespace rtb200

@@ -173,7 +173,7 @@ enum PtCounter : int {
     kCntShadowRays = 6,
     kCntAssigned = 7,   // free slots given camera samples this iteration
     kCntClass = 8,      // kCntClass + c: active paths of shading class c (KClassify)
-    kCntJobs = 11,      // entries of the job id list (written by the host)
+    kCntJobs = 12,      // entries of the job id list (written by the host)
     kCntCount = 16,
 };
 
@@ -264,10 +264,11 @@ struct PtQueues {
     int capacity;
 };
 
-// Shading classes: paths that escaped or hit Lambertian surfaces, GGX
-// conductors, smooth dielectrics.  KShade runs them as contiguous ranges so a
+// Shading classes: paths that hit Lambertian surfaces, GGX conductors, smooth
+// dielectrics (PtMatType), and those that escaped.  KShade runs them as contiguous ranges so a
 // warp shades one material model.
-constexpr int kShadeClasses = 3;
+constexpr int kShadeClasses = 4;
+constexpr int kClassEscaped = 3;
 
 struct PtFilm {
     float* pass;        // 3 floats per pixel, atomically accumulated this call
