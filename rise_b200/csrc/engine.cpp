@@ -199,8 +199,7 @@ int EngineCreate(rtb200_ctx* ctx, int capacity, rtb200_engine** out)
     const size_t c = (size_t)capacity;
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t at = off; off += Align(bytes); return at; };
-    const size_t oRo = take(16 * c), oRd = take(16 * c), oHit = take(16 * c), oThr = take(16 * c), oL = take(16 * c),
-                 oAux = take(16 * c), oMeta = take(16 * c), oMed = take(16 * c);
+    const size_t oRay = take(32 * c), oRad = take(32 * c), oState = take(32 * c), oHit = take(16 * c), oMed = take(16 * c);
     const size_t oQa = take(4 * c), oQan = take(4 * c), oQf = take(4 * c), oQfn = take(4 * c);
     const size_t oSh = take(sizeof(ShadowEntry) * 8 * c);   // up to 4 light + 4 sky samples per path
     const size_t oShd = take(4 * c * kShadeClasses);
@@ -219,10 +218,10 @@ int EngineCreate(rtb200_ctx* ctx, int capacity, rtb200_engine** out)
     // Only what is read before it is written: the paths' flags, and everything
     // past the per-path arrays.  In stream order: an earlier engine's work on
     // the block may still run.
-    cudaError_t ce = cudaMemsetAsync(b + oMeta, 0, 16 * c, ctx->stream);
+    cudaError_t ce = cudaMemsetAsync(b + oState, 0, 32 * c, ctx->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(b + oTab, 0, off - oTab, ctx->stream);
-    e->paths = PtPaths{(float4*)(b + oRo), (float4*)(b + oRd), (float4*)(b + oHit), (float4*)(b + oThr),
-                       (float4*)(b + oL), (float4*)(b + oAux), (uint4*)(b + oMeta), (int4*)(b + oMed)};
+    e->paths = PtPaths{(PathPair*)(b + oRay), (PathPair*)(b + oRad), (PathPair*)(b + oState), (float4*)(b + oHit),
+                       (int4*)(b + oMed)};
     e->queues = PtQueues{(int*)(b + oQa), (int*)(b + oQan), (int*)(b + oQf), (int*)(b + oQfn),
                          (ShadowEntry*)(b + oSh), (int*)(b + oCnt), (unsigned long long*)(b + oSmp),
                          (unsigned long long*)(b + oTr), (unsigned*)(b + oErr), (PtAssign*)(b + oAsg),

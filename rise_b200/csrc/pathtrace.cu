@@ -325,12 +325,13 @@ KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
         const int slot = valid ? Q.free_[i] : -1;
         int fin_job = -1;
         if (valid) {
-            const uint4 m = P.meta[slot];
+            float4 aux, meta;
+            LoadPair(P.state + slot, aux, meta);
+            const uint4 m = Bits(meta);
             if (m.z & kFlagFinishing) {
-                const float4 aux = P.aux[slot];
                 fin_job = __float_as_int(aux.z);
-                Splat(jobs[fin_job], P.L[slot], aux.x, m);
-                P.meta[slot].z = m.z & ~kFlagFinishing;
+                Splat(jobs[fin_job], P.rad[slot].b, aux.x, m);
+                SetFlags(P, slot, m.z & ~kFlagFinishing);
             }
         }
         // Finished samples, one atomic per job present in the warp.
@@ -397,13 +398,12 @@ KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
                                        ? J.set.lmin + (float)min((int)(uw * (float)J.set.num_wl), J.set.num_wl - 1) *
                                                           J.set.wl_step
                                        : J.set.lmin + uw * (J.set.lmax - J.set.lmin);
-                P.ray_o[slot] = make_float4(J.cam.pos[0], J.cam.pos[1], J.cam.pos[2], 0.0f);
-                P.ray_d[slot] = make_float4(d.x, d.y, d.z, __int_as_float(0x7f800000));
-                P.thr[slot] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-                P.L[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                P.aux[slot] = make_float4(hero, 0.0f, __int_as_float(jid), 0.0f);
-                P.meta[slot] = make_uint4(pixel, sample,
-                                          kFlagConsiderEmission | (J.set.single ? (0xeu << kTermShift) : 0u), key);
+                StorePair(P.ray + slot, make_float4(J.cam.pos[0], J.cam.pos[1], J.cam.pos[2], 0.0f),
+                          make_float4(d.x, d.y, d.z, __int_as_float(0x7f800000)));
+                StorePair(P.rad + slot, make_float4(1.0f, 1.0f, 1.0f, 1.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+                StorePair(P.state + slot, make_float4(hero, 0.0f, __int_as_float(jid), 0.0f),
+                          Floats(make_uint4(pixel, sample,
+                                            kFlagConsiderEmission | (J.set.single ? (0xeu << kTermShift) : 0u), key)));
                 got = true;
             }
         }
@@ -446,12 +446,13 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
             qi = got;
             slot = Q.active[qi];
             if (!UNIFORM) {
-                const PtScene& S = jobs[__float_as_int(P.aux[slot].z)].scene;
+                const PtScene& S = jobs[PathJob(P, slot)].scene;
                 nodes = (const NodeT*)S.nodes;
                 tris = S.tris;
                 ntri = S.ntri;
             }
-            const float4 o = P.ray_o[slot], d = P.ray_d[slot];
+            float4 o, d;
+            LoadPair(P.ray + slot, o, d);
             Ray r;
             r.o[0] = o.x; r.o[1] = o.y; r.o[2] = o.z; r.tmin = o.w;
             r.d[0] = d.x; r.d[1] = d.y; r.d[2] = d.z; r.tmax = d.w;
@@ -474,7 +475,7 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
 // Adds an unoccluded shadow entry's contribution to its path's radiance.
 __device__ __forceinline__ void AddShadow(const PtPaths& P, const ShadowEntry& e)
 {
-    float* l = reinterpret_cast<float*>(P.L + __float_as_int(e.d.w));
+    float* l = &P.rad[__float_as_int(e.d.w)].b.x;
     if (e.c.x != 0.0f) atomicAdd(l + 0, e.c.x);
     if (e.c.y != 0.0f) atomicAdd(l + 1, e.c.y);
     if (e.c.z != 0.0f) atomicAdd(l + 2, e.c.z);
@@ -505,7 +506,7 @@ KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
             qi = got;
             const ShadowEntry e = Q.shadow[qi];
             if (!UNIFORM) {
-                const PtScene& S = jobs[__float_as_int(P.aux[__float_as_int(e.d.w)].z)].scene;
+                const PtScene& S = jobs[PathJob(P, __float_as_int(e.d.w))].scene;
                 nodes = (const NodeT*)S.nodes;
                 tris = S.tris;
                 ntri = S.ntri;
@@ -621,7 +622,7 @@ KClassify(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
             const int hslot = __float_as_int(P.hit[slot].y);
             cls = kClassEscaped;
             if (hslot >= 0) {
-                const PtScene& S = jobs[__float_as_int(P.aux[slot].z)].scene;
+                const PtScene& S = jobs[PathJob(P, slot)].scene;
                 cls = S.mats[S.attr[hslot].mat & kAttrMatMask].type;
             }
         }
@@ -649,17 +650,18 @@ KEscape(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
         int slot = -1;
         if (valid) {
             slot = src[base + lane];
-            const float4 aux = P.aux[slot];
-            const uint4 m = P.meta[slot];
-            const float4 rd = P.ray_d[slot], thr = P.thr[slot];
-            float4 L = P.L[slot];
+            float4 aux, meta, thr, L;
+            LoadPair(P.state + slot, aux, meta);
+            LoadPair(P.rad + slot, thr, L);
+            const uint4 m = Bits(meta);
+            const float4 rd = P.ray[slot].b;
             const PtJobDev& J = jobs[__float_as_int(aux.z)];
             float lam[4];
             Wavelengths(aux.x, J.set.lmin, J.set.lmax, lam);
             AddSky<ENV>(J.scene, J.set, (int)(m.z & kFlagDepthMask), xyz(rd), aux.y, (m.z >> kTermShift) & 0xfu, lam,
                         thr, L);
-            P.L[slot] = L;
-            P.meta[slot].z = m.z | kFlagFinishing;
+            P.rad[slot].b = L;
+            SetFlags(P, slot, m.z | kFlagFinishing);
         }
         int* const queues[1] = {&Q.cnt[kCntFreeNext]};
         const int count[1] = {valid};
@@ -699,15 +701,15 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
         V3 p, nface;
         bool ng_flipped = false;
         if (valid) {
-            const float4 aux = P.aux[slot];
+            float4 aux, meta, ro, rd, thr, L;
+            LoadPair(P.state + slot, aux, meta);
+            LoadPair(P.ray + slot, ro, rd);
+            LoadPair(P.rad + slot, thr, L);
             const PtJobDev& J = jobs[__float_as_int(aux.z)];
             const PtScene& S = J.scene;
             const PtSettings& set = J.set;
-            uint4 m = P.meta[slot];
+            uint4 m = Bits(meta);
             const float4 h = P.hit[slot];
-            const float4 ro = P.ray_o[slot], rd = P.ray_d[slot];
-            float4 thr = P.thr[slot];
-            float4 L = P.L[slot];
             const int depth = (int)(m.z & kFlagDepthMask);
             // Random numbers: hash key or Sobol seed in meta.w, sample index in meta.y.
             VertexRng rng{m.w, m.y, depth, set.sampler, 0u, 0u, 0u};
@@ -1194,21 +1196,23 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class)
                 if (depth + 1 >= set.max_depth) break;
                 thr = make_float4(thr.x * kray.x, thr.y * kray.y, thr.z * kray.z, thr.w * kray.w);
                 const V3 no = OffsetRay(p, nface, nd);
-                P.ray_o[slot] = make_float4(no.x, no.y, no.z, 0.0f);
-                P.ray_d[slot] = make_float4(nd.x, nd.y, nd.z, __int_as_float(0x7f800000));
-                P.thr[slot] = thr;
-                P.aux[slot] = make_float4(aux.x, npdf, aux.z, __uint_as_float(bounces));
+                StorePair(P.ray + slot, make_float4(no.x, no.y, no.z, 0.0f),
+                          make_float4(nd.x, nd.y, nd.z, __int_as_float(0x7f800000)));
                 m.z = (m.z & ~(kFlagDepthMask | kFlagSpecular)) | (unsigned)(depth + 1) | nflags;
                 if (media_changed) {
                     P.media[slot] = med;
                     m.z = med.x >= 0 ? (m.z | kFlagInMedium) : (m.z & ~kFlagInMedium);
                 }
-                P.meta[slot].z = m.z;
+                StorePair(P.state + slot, make_float4(aux.x, npdf, aux.z, __uint_as_float(bounces)), Floats(m));
                 cont = true;
             } while (false);
 
-            P.L[slot] = L;
-            if (!cont) P.meta[slot].z = m.z | kFlagFinishing;
+            if (cont) {
+                StorePair(P.rad + slot, thr, L);
+            } else {
+                P.rad[slot].b = L;
+                SetFlags(P, slot, m.z | kFlagFinishing);
+            }
         }
         int* const queues[3] = {&Q.cnt[kCntShadow], &Q.cnt[kCntActiveNext], &Q.cnt[kCntFreeNext]};
         const int count[3] = {__popc(events), cont, valid && !cont};

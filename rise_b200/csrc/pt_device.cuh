@@ -314,6 +314,35 @@ __device__ __forceinline__ float PowerHeuristic(float a, float b)
     return a2 / (a2 + b * b);
 }
 
+// A path's pair in one access.
+__device__ __forceinline__ void LoadPair(const PathPair* p, float4& a, float4& b)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void StorePair(PathPair* p, const float4& a, const float4& b)
+{
+    asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
+                 "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w), "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ uint4 Bits(const float4& v)
+{
+    return make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+}
+__device__ __forceinline__ float4 Floats(const uint4& v)
+{
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+// The path's job and its flags alone.
+__device__ __forceinline__ int PathJob(const PtPaths& P, int slot) { return __float_as_int(P.state[slot].a.z); }
+__device__ __forceinline__ void SetFlags(const PtPaths& P, int slot, unsigned flags)
+{
+    P.state[slot].b.z = __uint_as_float(flags);
+}
+
 // Appends to up to four queues at once, called by a whole warp: a lane adds
 // n[q] entries to queue q and gets its first index in at[q].  The counts
 // (below 1024 a warp, 256 with four queues) are summed in one packed scan and

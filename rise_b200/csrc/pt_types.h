@@ -225,14 +225,22 @@ RTB_HD unsigned OctEncode(float x, float y, float z)
     return ((unsigned)qu & 0xffffu) | ((unsigned)qv << 16);
 }
 
+// Path state comes in pairs that are read and written together: a pair is one
+// 32-byte sector and one access.  A path's slot is anywhere in the pool, and 16
+// bytes alone cost a sector all the same (800k-triangle scene at 8 spp, whose
+// pool of 2^21 paths does not fit the L2: 29.0 -> 27.1 ms; 2^19 paths 3.13 ->
+// 3.03 ms on the Cornell box).
+struct alignas(32) PathPair {
+    float4 a, b;
+};
+
 struct PtPaths {
-    float4* ray_o;   // origin, tmin
-    float4* ray_d;   // direction, tmax
-    float4* hit;     // t, leaf slot (int bits, -1 miss), a, b
-    float4* thr;     // throughput per wavelength
-    float4* L;       // radiance per wavelength
-    float4* aux;     // x hero wavelength, y bsdf pdf
-    uint4* meta;     // x pixel, y sample, z flags, w rng key
+    PathPair* ray;     // a origin, tmin; b direction, tmax
+    PathPair* rad;     // per wavelength: a throughput, b radiance
+    // a: x hero wavelength, y bsdf pdf, z job, w bounce counts; b (bits): x
+    // pixel, y sample, z flags, w rng key
+    PathPair* state;
+    float4* hit;       // t, leaf slot (int bits, -1 miss), a, b
     // Index-of-refraction stack (Utilities/IORStack.h): the dielectric
     // meshes the path is inside, innermost last, -1 past the top; read only
     // when meta.z has kFlagInMedium (an empty stack otherwise).
