@@ -430,14 +430,14 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
     const NodeT* nodes = UNIFORM ? (const NodeT*)us.nodes : nullptr;
     const GpuTri* tris = UNIFORM ? us.tris : nullptr;
     int ntri = UNIFORM ? us.ntri : 0;
-    __shared__ int sstack[kTraceStack * kTraceBlock];
+    __shared__ int sstack[kStackRows * kTraceBlock];
     int spill[SPILL ? kTraceSpill : 1];
-    const TraceStack stk{sstack + threadIdx.x, spill};
+    const TraceStack stk = MakeStack(sstack + threadIdx.x, spill);
     const unsigned n = (unsigned)Q.cnt[kCntActive];
     const unsigned chunk = FeedChunk(n, (gridDim.x * blockDim.x) >> 5);
     WarpFeed feed = FeedStart(n, chunk);
     TraceState s;
-    if (COOP) s.sp = 0;
+    if (COOP) s.sp = stk.bottom, s.over = 0;
     int qi = -1;
     int slot = -1;
     for (;;) {
@@ -456,18 +456,18 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
             Ray r;
             r.o[0] = o.x; r.o[1] = o.y; r.o[2] = o.z; r.tmin = o.w;
             r.d[0] = d.x; r.d[1] = d.y; r.d[2] = d.z; r.tmax = d.w;
-            StartRay(s, r);
+            StartRay(s, r, stk.bottom);
         }
         const unsigned live = __ballot_sync(kFull, qi >= 0);
         if (!live) return;
-        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, live)) break;
+        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, stk, live)) break;
         if (qi >= 0 && TraceRound<NodeT, false, SPILL, kPathLeaves>(s, nodes, tris, ntri, stk, Q.err)) {
             P.hit[slot] = make_float4(s.best, __int_as_float(s.bestSlot), s.ba, s.bb);
             qi = -1;
         }
     }
     if (COOP) {
-        CoopFinish<NodeT, false, SPILL>(s, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
+        CoopFinish<NodeT, false, SPILL>(s, stk, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
         if (qi >= 0) P.hit[slot] = make_float4(s.best, __int_as_float(s.bestSlot), s.ba, s.bb);
     }
 }
@@ -491,14 +491,14 @@ KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
     const NodeT* nodes = UNIFORM ? (const NodeT*)us.nodes : nullptr;
     const GpuTri* tris = UNIFORM ? us.tris : nullptr;
     int ntri = UNIFORM ? us.ntri : 0;
-    __shared__ int sstack[kTraceStack * kTraceBlock];
+    __shared__ int sstack[kStackRows * kTraceBlock];
     int spill[SPILL ? kTraceSpill : 1];
-    const TraceStack stk{sstack + threadIdx.x, spill};
+    const TraceStack stk = MakeStack(sstack + threadIdx.x, spill);
     const unsigned n = (unsigned)Q.cnt[kCntShadow];
     const unsigned chunk = FeedChunk(n, (gridDim.x * blockDim.x) >> 5);
     WarpFeed feed = FeedStart(n, chunk);
     TraceState s;
-    if (COOP) s.sp = 0;
+    if (COOP) s.sp = stk.bottom, s.over = 0;
     int qi = -1;
     for (;;) {
         const int got = FeedTake(feed, qi < 0, n, chunk, (unsigned*)(Q.trace_ctr + 1));
@@ -514,18 +514,18 @@ KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
             Ray r;
             r.o[0] = e.o.x; r.o[1] = e.o.y; r.o[2] = e.o.z; r.tmin = 0.0f;
             r.d[0] = e.d.x; r.d[1] = e.d.y; r.d[2] = e.d.z; r.tmax = e.o.w;
-            StartRay(s, r);
+            StartRay(s, r, stk.bottom);
         }
         const unsigned live = __ballot_sync(kFull, qi >= 0);
         if (!live) return;
-        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, live)) break;
+        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, stk, live)) break;
         if (qi >= 0 && TraceRound<NodeT, true, SPILL, kPathLeaves>(s, nodes, tris, ntri, stk, Q.err)) {
             if (s.bestSlot < 0) AddShadow(P, Q.shadow[qi]);
             qi = -1;
         }
     }
     if (COOP) {
-        CoopFinish<NodeT, true, SPILL>(s, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
+        CoopFinish<NodeT, true, SPILL>(s, stk, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
         if (qi >= 0 && s.bestSlot < 0) AddShadow(P, Q.shadow[qi]);
     }
 }

@@ -61,29 +61,29 @@ KTrace(const NodeT* __restrict__ nodes, const GpuTri* __restrict__ tris,
        const rtb200_ray* __restrict__ rays, unsigned n, int ntri, rtb200_hit* __restrict__ hits,
        uint8_t* __restrict__ occ, unsigned chunk, unsigned* counter, unsigned* err)
 {
-    __shared__ int sstack[kTraceStack * kTraceBlock];
+    __shared__ int sstack[kStackRows * kTraceBlock];
     int spill[SPILL ? kTraceSpill : 1];
-    const TraceStack stk{sstack + threadIdx.x, spill};
+    const TraceStack stk = MakeStack(sstack + threadIdx.x, spill);
     WarpFeed feed = FeedStart(n, chunk);
     TraceState s;
-    if (COOP) s.sp = 0;
+    if (COOP) s.sp = stk.bottom, s.over = 0;
     int ray = -1;
     for (;;) {
         const int got = FeedTake(feed, ray < 0, n, chunk, counter);
         if (got >= 0) {
             ray = got;
-            StartRay(s, LoadRay(rays, ray));
+            StartRay(s, LoadRay(rays, ray), stk.bottom);
         }
         const unsigned live = __ballot_sync(kFull, ray >= 0);
         if (!live) return;
-        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, live)) break;
+        if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, stk, live)) break;
         if (ray >= 0 && TraceRound<NodeT, ANY, SPILL, kCastLeaves>(s, nodes, tris, ntri, stk, err)) {
             StoreAnswer<ANY>(s, tris, rays, ray, hits, occ);
             ray = -1;
         }
     }
     if (COOP) {
-        CoopFinish<NodeT, ANY, SPILL>(s, ray >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), err);
+        CoopFinish<NodeT, ANY, SPILL>(s, stk, ray >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), err);
         if (ray >= 0) StoreAnswer<ANY>(s, tris, rays, ray, hits, occ);
     }
 }
