@@ -205,7 +205,7 @@ int EngineCreate(rtb200_ctx* ctx, int capacity, rtb200_engine** out)
     const size_t oShd = take(4 * c * kShadeClasses);
     const size_t oTab = take(sizeof(PtJobDev) * kMaxJobs), oIds = take(4 * kMaxJobs),
                  oCtr = take(8 * 2 * kMaxJobs);
-    const size_t oCnt = take(4 * kCntCount), oTr = take(8 * 2), oSmp = take(8), oErr = take(4),
+    const size_t oCnt = take(4 * kCntCount), oTr = take(8 * 4), oSmp = take(8), oErr = take(4),
                  oAsg = take(sizeof(PtAssign) * kMaxJobs);
     // The pool and the pinned tables come back from the context when an engine
     // before this one had the same capacity: allocating, clearing and freeing

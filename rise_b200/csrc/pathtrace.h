@@ -29,7 +29,7 @@ struct PtLaunch {
     cudaEvent_t fork, join[2];
 };
 
-// One wavefront iteration (rotate counters, regenerate, extend, shade, connect),
+// One wavefront iteration (connect the last one, rotate counters, regenerate, extend, shade),
 // asynchronous on `st`.  The caller swaps queues.active/active_next and
 // queues.free_/free_next after each call.
 cudaError_t PtIteration(const PtLaunch& L, int iter, cudaStream_t st);

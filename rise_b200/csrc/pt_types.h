@@ -165,7 +165,7 @@ struct ShadowEntry {
 // Counters in device memory.
 enum PtCounter : int {
     kCntActive = 0,     // paths to extend this iteration
-    kCntActiveNext = 1,
+    kCntFreshRays = 1,  // first of this iteration's new paths in the active queue
     kCntFree = 2,       // finished / empty slots to regenerate
     kCntFreeNext = 3,
     kCntShadow = 4,
@@ -174,6 +174,10 @@ enum PtCounter : int {
     kCntAssigned = 7,   // free slots given camera samples this iteration
     kCntClass = 8,      // kCntClass + c: active paths of shading class c (KClassify)
     kCntJobs = 12,      // entries of the job id list (written by the host)
+    // Paths that continue: kCntNext + p is appended to by an iteration of parity
+    // p and read by the next one, whose KExtend may still read it while KAssign
+    // prepares the counters of the iteration after.
+    kCntNext = 14,
     kCntCount = 16,
 };
 
@@ -265,7 +269,7 @@ struct PtQueues {
     ShadowEntry* shadow;
     int* cnt;           // PtCounter
     unsigned long long* sample_ctr;
-    unsigned long long* trace_ctr;   // [2]: extend, connect
+    unsigned long long* trace_ctr;   // feeds: connect, extend new, extend continuing of parity 0 and 1
     unsigned* err;
     PtAssign* assign;                // [max jobs], written by KAssign
     int* shade;                      // [kShadeClasses][capacity]: active slots by shading class
