@@ -123,13 +123,20 @@ int EnsureStage(rtb200_scene* s, size_t in_bytes, size_t out_bytes)
 // alternate between two trace streams (ctx->stream, ctx->trace2), each launch
 // with its own work counter, so one chunk's blocks start while the previous
 // chunk's last rays finish instead of the device idling in every launch's tail.
+// A download is issued after the next chunk's upload and launch: from and to
+// pageable memory a copy holds the calling thread, which a download of chunk k
+// does until its trace is done (500,000 rays: 1869 -> 1331 us).
 // `trace(d_in, m, d_out, counter, stream)` launches the kernel on m staged rays.
 template <class Trace>
 cudaError_t PipelinedCast(rtb200_scene* s, const rtb200_ray* rays, int64_t n, void* out, size_t out_bytes_per_ray,
                           int& rc, Trace trace)
 {
     rtb200_ctx* ctx = s->ctx;
-    const int64_t chunk = std::max<int64_t>(std::min<int64_t>(n, int64_t(1) << 18), (n + 7) / 8);
+    // Two halves from 2^17 rays, so that one's upload runs beside the other's
+    // trace (250,001 rays from pageable memory: 982 us in one piece, 791 in two),
+    // then pieces of 2^18, at most eight.
+    constexpr int64_t kWhole = int64_t(1) << 17, kPiece = int64_t(1) << 18;
+    const int64_t chunk = n <= kWhole ? n : std::max(std::min((n + 1) / 2, kPiece), (n + 7) / 8);
     const int nbuf = n > chunk ? 2 : 1;
     rc = EnsureStage(s, (size_t)nbuf * chunk * sizeof(rtb200_ray), (size_t)nbuf * chunk * out_bytes_per_ray);
     if (rc) return cudaSuccess;
@@ -142,24 +149,32 @@ cudaError_t PipelinedCast(rtb200_scene* s, const rtb200_ray* rays, int64_t n, vo
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->copy_in, ctx->ev_trace[0], 0);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ts[1], ctx->ev_trace[0], 0);
     const int64_t nchunks = (n + chunk - 1) / chunk;
-    for (int64_t k = 0; k < nchunks && e == cudaSuccess; ++k) {
-        const int b = (int)(k & 1);
-        const int64_t off = k * chunk, m = std::min(chunk, n - off);
-        rtb200_ray* d_in = (rtb200_ray*)s->d_in + b * chunk;
-        char* d_out = (char*)s->d_out + (size_t)b * chunk * out_bytes_per_ray;
-        if (k >= 2) e = cudaStreamWaitEvent(ctx->copy_in, ctx->ev_trace[b], 0);   // chunk k-2 traced
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d_in, rays + off, (size_t)m * sizeof(rtb200_ray), cudaMemcpyHostToDevice, ctx->copy_in);
-        if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_up[b], ctx->copy_in);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(ts[b], ctx->ev_up[b], 0);
-        if (e == cudaSuccess && k >= 2) e = cudaStreamWaitEvent(ts[b], ctx->ev_down[b], 0);   // chunk k-2 downloaded
-        if (e == cudaSuccess) e = trace(d_in, m, d_out, counter[b], ts[b]);
-        if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_trace[b], ts[b]);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->copy_out, ctx->ev_trace[b], 0);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync((char*)out + (size_t)off * out_bytes_per_ray, d_out, (size_t)m * out_bytes_per_ray,
-                                cudaMemcpyDeviceToHost, ctx->copy_out);
-        if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_down[b], ctx->copy_out);
+    for (int64_t k = 0; k <= nchunks && e == cudaSuccess; ++k) {
+        if (k < nchunks) {
+            const int b = (int)(k & 1);
+            const int64_t off = k * chunk, m = std::min(chunk, n - off);
+            rtb200_ray* d_in = (rtb200_ray*)s->d_in + b * chunk;
+            char* d_out = (char*)s->d_out + (size_t)b * chunk * out_bytes_per_ray;
+            if (k >= 2) e = cudaStreamWaitEvent(ctx->copy_in, ctx->ev_trace[b], 0);   // chunk k-2 traced
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(d_in, rays + off, (size_t)m * sizeof(rtb200_ray), cudaMemcpyHostToDevice,
+                                    ctx->copy_in);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_up[b], ctx->copy_in);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(ts[b], ctx->ev_up[b], 0);
+            if (e == cudaSuccess && k >= 2) e = cudaStreamWaitEvent(ts[b], ctx->ev_down[b], 0);   // k-2 downloaded
+            if (e == cudaSuccess) e = trace(d_in, m, d_out, counter[b], ts[b]);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_trace[b], ts[b]);
+        }
+        if (k >= 1 && e == cudaSuccess) {
+            const int b = (int)((k - 1) & 1);
+            const int64_t off = (k - 1) * chunk, m = std::min(chunk, n - off);
+            const char* d_out = (const char*)s->d_out + (size_t)b * chunk * out_bytes_per_ray;
+            e = cudaStreamWaitEvent(ctx->copy_out, ctx->ev_trace[b], 0);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync((char*)out + (size_t)off * out_bytes_per_ray, d_out, (size_t)m * out_bytes_per_ray,
+                                    cudaMemcpyDeviceToHost, ctx->copy_out);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_down[b], ctx->copy_out);
+        }
     }
     // Later work on ctx->stream waits for both trace streams and the downloads.
     if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_trace[1], ts[1]);

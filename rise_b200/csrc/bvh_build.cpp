@@ -683,8 +683,10 @@ void EncodeTriangles(const float* tri9, const BuiltBVH& b, std::vector<GpuTri>& 
     for (const Node4& n : b.nodes4)
         for (int i = 0; i < n.nchild; ++i)
             if (n.count[i] > 0) {
-                const size_t at = (size_t)n.child[i] + n.count[i] - 1;
-                out[at] = EncodeTriangle(tri9, b.prims[at], true);
+                GpuTri& t = out[(size_t)n.child[i] + n.count[i] - 1];
+                t.x.w |= INT32_MIN;
+                t.y.w |= INT32_MIN;
+                t.z.w |= INT32_MIN;
             }
 }
 
