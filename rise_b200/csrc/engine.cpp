@@ -168,6 +168,8 @@ PtLaunch MakeLaunch(const rtb200_engine* e)
     }
     if (L.classify) L.shade_class = -1;
     L.scene = L.uniform ? e->h_table[e->active[0]].scene : PtScene{};
+    L.one = false;
+    L.job = e->active.size() == 1 ? e->h_table[e->active[0]] : PtJobDev{};
     L.paths = e->paths;
     L.queues = e->queues;
     L.sms = e->ctx->num_sms;
@@ -390,6 +392,7 @@ int EngineStep(rtb200_engine* e, int iterations, bool graph)
     } else {
         // Direct launches; an even count keeps the queue buffers where the
         // captured graph expects them.
+        L.one = e->active.size() == 1;
         const int n = ((iterations + 1) / 2) * 2;
         for (int k = 0; k < n && err == cudaSuccess; ++k) {
             err = PtIteration(L, e->iter++, st);

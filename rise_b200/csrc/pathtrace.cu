@@ -194,6 +194,18 @@ __device__ __forceinline__ void Splat(const PtJobDev& J, float4 L, float hero, u
 
 // ---- kernels ---------------------------------------------------------------
 
+// A path's job: the kernel argument where the engine renders one job (ONE),
+// whose scene, camera and settings are then operands from the constant bank,
+// else an entry of the job table, each use of which is a load (Cornell box at 16
+// spp 2.87 ms from the table, 2.77 from the argument; adaptive 200 x 150 image
+// 3.53 and 3.38).
+template <bool ONE>
+__device__ __forceinline__ const PtJobDev& JobOf(const PtJobDev* __restrict__ jobs, const PtJobDev& one, int jid)
+{
+    if constexpr (ONE) return one;
+    else return jobs[jid];
+}
+
 // First in every kernel of an iteration: waits for the stream's previous kernel
 // to end, when this one was launched ahead of that (Chain below).  The launch
 // latency is then off the path: a 120 x 80 image at 4 spp 1.95 -> 1.78 ms, the
@@ -321,8 +333,9 @@ KAssign(const PtJobDev* __restrict__ jobs, const int* __restrict__ ids, PtQueues
     else if (threadIdx.x < 32) AssignJobs<true>(jobs, ids, Q, iter, njobs, n);
 }
 
+template <bool ONE>
 __global__ void __launch_bounds__(kShadeBlock)
-KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
+KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, const __grid_constant__ PtJobDev one)
 {
     ChainStart();
     const int njobs = Q.cnt[kCntJobs];
@@ -342,13 +355,13 @@ KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
             const uint4 m = Bits(meta);
             if (m.z & kFlagFinishing) {
                 fin_job = __float_as_int(aux.z);
-                Splat(jobs[fin_job], P.rad[slot].b, aux.x, m);
+                Splat(JobOf<ONE>(jobs, one, fin_job), P.rad[slot].b, aux.x, m);
                 SetFlags(P, slot, m.z & ~kFlagFinishing);
             }
         }
         // Finished samples, one atomic per job present in the warp.
         const unsigned grp = __match_any_sync(kFull, fin_job);
-        if (fin_job >= 0 && lane == __ffs(grp) - 1) atomicAdd(jobs[fin_job].done_ctr, (unsigned long long)__popc(grp));
+        if (fin_job >= 0 && lane == __ffs(grp) - 1) atomicAdd(JobOf<ONE>(jobs, one, fin_job).done_ctr, (unsigned long long)__popc(grp));
         // New camera samples: free entry i < nassigned belongs to the job
         // whose assigned range holds it (KAssign).
         bool got = false;
@@ -360,7 +373,7 @@ KRegen(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
             }
             const PtAssign a = Q.assign[lo];
             const int jid = a.jid;
-            const PtJobDev& J = jobs[jid];
+            const PtJobDev& J = JobOf<ONE>(jobs, one, jid);
             const unsigned long long g = a.base + (unsigned long long)(i - a.off);
             {   // PinholeCamera::GenerateRay (Cameras/PinholeCamera.cpp:182-210)
                 // 64-bit division only where the request needs it.
@@ -662,9 +675,9 @@ KClassify(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
 // Escaped paths after KClassify: the sky's radiance, and the end of the path.
 // In KShade<0> they left half of the lanes of a Lambertian warp idle (16 of 32
 // active): 189 us an iteration of the 800k-triangle scene, now 109 and 24.
-template <bool ENV>
+template <bool ENV, bool ONE>
 __global__ void __launch_bounds__(kShadeBlock)
-KEscape(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
+KEscape(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, const __grid_constant__ PtJobDev one)
 {
     ChainStart();
     const int n = Q.cnt[kCntClass + kClassEscaped];
@@ -680,7 +693,7 @@ KEscape(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
             LoadPair(P.rad + slot, thr, L);
             const uint4 m = Bits(meta);
             const float4 rd = P.ray[slot].b;
-            const PtJobDev& J = jobs[__float_as_int(aux.z)];
+            const PtJobDev& J = JobOf<ONE>(jobs, one, __float_as_int(aux.z));
             float lam[4];
             Wavelengths(aux.x, J.set.lmin, J.set.lmax, lam);
             AddSky<ENV>(J.scene, J.set, (int)(m.z & kFlagDepthMask), xyz(rd), aux.y, (m.z >> kTermShift) & 0xfu, lam,
@@ -702,9 +715,10 @@ KEscape(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
 // KClassify's queue of that class (from_class, no escaped ones) or, for scenes
 // of one class, straight from the active queue.  CLS = -1 shades any material from the active queue.
 // ENV: compiled with the image-environment code (some job's scene has one).
-template <int CLS, bool ENV>
+template <int CLS, bool ENV, bool ONE>
 __global__ void __launch_bounds__(kShadeBlock, CLS == 1 || CLS < 0 ? 2 : 3)
-KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class, int parity)
+KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class, int parity,
+       const __grid_constant__ PtJobDev one)
 {
     ChainStart();
     const int n = (CLS >= 0 && from_class) ? Q.cnt[kCntClass + (CLS < 0 ? 0 : CLS)] : Q.cnt[kCntActive];
@@ -731,7 +745,7 @@ KShade(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, int from_class,
             LoadPair(P.state + slot, aux, meta);
             LoadPair(P.ray + slot, ro, rd);
             LoadPair(P.rad + slot, thr, L);
-            const PtJobDev& J = jobs[__float_as_int(aux.z)];
+            const PtJobDev& J = JobOf<ONE>(jobs, one, __float_as_int(aux.z));
             const PtScene& S = J.scene;
             const PtSettings& set = J.set;
             uint4 m = Bits(meta);
@@ -1448,8 +1462,9 @@ template <int CLS>
 void LaunchShade(const PtLaunch& L, int from_class, int parity, cudaStream_t st)
 {
     const int grid = L.sms * 8;
-    if (L.env_image) Chain(KShade<CLS, true>, grid, kShadeBlock, st, L.jobs, L.paths, L.queues, from_class, parity);
-    else Chain(KShade<CLS, false>, grid, kShadeBlock, st, L.jobs, L.paths, L.queues, from_class, parity);
+    auto* kernel = L.env_image ? (L.one ? KShade<CLS, true, true> : KShade<CLS, true, false>)
+                               : (L.one ? KShade<CLS, false, true> : KShade<CLS, false, false>);
+    Chain(kernel, grid, kShadeBlock, st, L.jobs, L.paths, L.queues, from_class, parity, L.job);
 }
 
 cudaError_t PtIteration(const PtLaunch& L, int iter, cudaStream_t st)
@@ -1470,7 +1485,7 @@ cudaError_t PtIteration(const PtLaunch& L, int iter, cudaStream_t st)
     }
     LaunchTrace(L, rays, TraceKind::Connect, parity);
     Chain(KAssign, 1, kPtMaxJobs, rays, L.jobs, L.ids, L.queues, iter);
-    Chain(KRegen, shadeGrid, kShadeBlock, rays, L.jobs, L.paths, L.queues);
+    Chain(L.one ? KRegen<true> : KRegen<false>, shadeGrid, kShadeBlock, rays, L.jobs, L.paths, L.queues, L.job);
     LaunchTrace(L, rays, L.coop ? TraceKind::ExtendNew : TraceKind::Extend, parity);
     if (L.coop) {
         cudaEventRecord(L.join[0], rays);
@@ -1485,10 +1500,12 @@ cudaError_t PtIteration(const PtLaunch& L, int iter, cudaStream_t st)
         cudaStreamWaitEvent(L.side[1], L.fork, 0);
         LaunchShade<1>(L, 1, parity, st);
         LaunchShade<0>(L, 1, parity, L.side[0]);
-        if (L.env_image) Chain(KEscape<true>, shadeGrid, kShadeBlock, L.side[1], L.jobs, L.paths, L.queues);
-        else Chain(KEscape<false>, shadeGrid, kShadeBlock, L.side[1], L.jobs, L.paths, L.queues);
+        auto* escape = L.env_image ? (L.one ? KEscape<true, true> : KEscape<true, false>)
+                                   : (L.one ? KEscape<false, true> : KEscape<false, false>);
+        Chain(escape, shadeGrid, kShadeBlock, L.side[1], L.jobs, L.paths, L.queues, L.job);
         // Dielectrics shade no next events.
-        Chain(KShade<2, false>, shadeGrid, kShadeBlock, L.side[1], L.jobs, L.paths, L.queues, 1, parity);
+        Chain(L.one ? KShade<2, false, true> : KShade<2, false, false>, shadeGrid, kShadeBlock, L.side[1], L.jobs,
+              L.paths, L.queues, 1, parity, L.job);
         for (int k = 0; k < 2; ++k) {
             cudaEventRecord(L.join[k], L.side[k]);
             cudaStreamWaitEvent(st, L.join[k], 0);

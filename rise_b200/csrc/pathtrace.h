@@ -21,6 +21,8 @@ struct PtLaunch {
     bool coop;         // some job's BVH is deep enough that a warp's last rays are worth finishing together
     bool env_image;    // some job's scene has an image environment (shading kernels carry its code)
     PtScene scene;
+    bool one;          // the engine renders one job, `job`, and the launch is not captured
+    PtJobDev job;
     PtPaths paths;
     PtQueues queues;
     int sms;
