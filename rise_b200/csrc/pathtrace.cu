@@ -35,6 +35,12 @@ constexpr int kShadeBlock = 256;
 // Leaves tested per lane per traversal round in KExtend / KConnect (measured
 // best for the path tracer's mixed secondary and shadow rays).
 constexpr int kPathLeaves = 1;
+// Lanes that may lack a leaf when the descent stops (raycast.cu).  Over deep
+// trees (COOP) 16: 800k-triangle scene at 8 spp 25.8 ms with 12, 24.8 with 16 and
+// 18, 26.1 with 24; over small ones 12: Cornell box at 16 spp 2.76, 2.77, 2.78,
+// 2.81 ms.
+template <bool COOP>
+constexpr int kPathLack = COOP ? 16 : 12;
 constexpr float kInv4Pi = 0.07957747154594767f;
 
 // ---- light BVH -------------------------------------------------------------
@@ -496,7 +502,7 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us, in
         const unsigned live = __ballot_sync(kFull, qi >= 0);
         if (!live) return;
         if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, stk, live)) break;
-        if (qi >= 0 && TraceRound<NodeT, false, SPILL, kPathLeaves>(s, nodes, tris, ntri, stk, Q.err)) {
+        if (qi >= 0 && TraceRound<NodeT, false, SPILL, kPathLeaves, kPathLack<COOP>>(s, nodes, tris, ntri, stk, Q.err)) {
             P.hit[slot] = make_float4(s.best, __int_as_float(s.bestSlot), s.ba, s.bb);
             qi = -1;
         }
@@ -555,7 +561,7 @@ KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
         const unsigned live = __ballot_sync(kFull, qi >= 0);
         if (!live) return;
         if (COOP && __popc(live) <= kCoopRays && FeedDry(feed) && CoopReady<SPILL>(s, stk, live)) break;
-        if (qi >= 0 && TraceRound<NodeT, true, SPILL, kPathLeaves>(s, nodes, tris, ntri, stk, Q.err)) {
+        if (qi >= 0 && TraceRound<NodeT, true, SPILL, kPathLeaves, kPathLack<COOP>>(s, nodes, tris, ntri, stk, Q.err)) {
             if (s.bestSlot < 0) AddShadow(P, Q.shadow[qi]);
             qi = -1;
         }

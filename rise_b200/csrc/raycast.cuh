@@ -517,13 +517,8 @@ __device__ __forceinline__ int Pop(TraceState& s, const TraceStack& st)
     return LoadShared(s.sp);
 }
 
-// Lanes of a warp that may still lack a postponed leaf when the descent
-// stops: waiting for the last few lanes to find one left most lanes idle.
-// 8 and 16 lanes were 2 to 4 % slower on a 1M-triangle soup.
-constexpr int kDescentLanes = 12;
-
 // One round of while-while traversal for every active lane: descend internal
-// nodes until fewer than kDescentLanes active lanes still lack a postponed
+// nodes until fewer than LACK active lanes still lack a postponed
 // leaf (or have run out of nodes), then test at most LEAVES leaves per lane
 // as one flat walk over their triangles; a leaf met after that is kept for the
 // next round, whose descent starts with it.  Measured on incoherent rays
@@ -532,7 +527,7 @@ constexpr int kDescentLanes = 12;
 // the leaf loop and 42 % in the descent; the cap, the flat walk and the early
 // stop together trace 70 % more rays per second.  ANY: stop at the first
 // accepted hit.  Returns true when this lane's ray is finished.
-template <class NodeT, bool ANY, bool SPILL, int LEAVES>
+template <class NodeT, bool ANY, bool SPILL, int LEAVES, int LACK>
 __device__ __forceinline__ bool TraceRound(TraceState& s, const NodeT* __restrict__ nodes,
                                            const GpuTri* __restrict__ tris, int ntri, const TraceStack& stk, unsigned* err)
 {
@@ -583,7 +578,7 @@ __device__ __forceinline__ bool TraceRound(TraceState& s, const NodeT* __restric
             s.leaf = s.node;
             s.node = Pop<SPILL>(s, stk);
         }
-        if (__popc(__ballot_sync(__activemask(), s.leaf == kEmpty)) < kDescentLanes) break;
+        if (__popc(__ballot_sync(__activemask(), s.leaf == kEmpty)) < LACK) break;
     }
     // Test leaves: one walk over the triangles of up to LEAVES leaves.
     int nleaf = 0;
