@@ -169,8 +169,8 @@ cudaError_t LaunchCastClosest(const rtb200_scene* s, const rtb200_ray* d_rays, i
                               rtb200_hit* d_hits, cudaStream_t stream);
 cudaError_t LaunchCastAny(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n,
                           uint8_t* d_occ, cudaStream_t stream);
-// Closest-hit launch with caller-provided scratch (work counter and error
-// word); clears nothing itself.
+// Launches with caller-provided scratch: the work counter, cleared here when the
+// batch needs it, and the error word, which is not.
 cudaError_t LaunchCastAnyScratch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n, uint8_t* d_occ,
                                  unsigned long long* counter, unsigned* err, cudaStream_t stream);
 cudaError_t LaunchCastClosestScratch(const rtb200_scene* s, const rtb200_ray* d_rays, int64_t n,
