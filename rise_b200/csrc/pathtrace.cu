@@ -190,10 +190,7 @@ __device__ __forceinline__ void Splat(const PtJobDev& J, float4 L, float hero, u
             if (fabsf(dx) > hw) continue;
             const float w = S.filt_norm * expf(-(dx * dx + dy * dy) * S.filt_inv2s2);
             float* f = J.film + 4 * ((size_t)qy * W + qx);
-            if (X != 0.0f) atomicAdd(f + 0, X * w);
-            if (Y != 0.0f) atomicAdd(f + 1, Y * w);
-            if (Z != 0.0f) atomicAdd(f + 2, Z * w);
-            atomicAdd(f + 3, w);
+            AtomicAdd4(f, X * w, Y * w, Z * w, w);
         }
     }
 }
@@ -517,6 +514,11 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us, in
 __device__ __forceinline__ void AddShadow(const PtPaths& P, const ShadowEntry& e)
 {
     float* l = &P.rad[__float_as_int(e.d.w)].b.x;
+    // One wavelength's contribution, or a sample that all four share.
+    if ((e.c.x != 0.0f) + (e.c.y != 0.0f) + (e.c.z != 0.0f) + (e.c.w != 0.0f) > 1) {
+        AtomicAdd4(l, e.c.x, e.c.y, e.c.z, e.c.w);
+        return;
+    }
     if (e.c.x != 0.0f) atomicAdd(l + 0, e.c.x);
     if (e.c.y != 0.0f) atomicAdd(l + 1, e.c.y);
     if (e.c.z != 0.0f) atomicAdd(l + 2, e.c.z);
@@ -680,7 +682,8 @@ KClassify(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q)
 
 // Escaped paths after KClassify: the sky's radiance, and the end of the path.
 // In KShade<0> they left half of the lanes of a Lambertian warp idle (16 of 32
-// active): 189 us an iteration of the 800k-triangle scene, now 109 and 24.
+// active): 189 us an iteration of the 800k-triangle scene together, 109 and 24
+// apart.
 template <bool ENV, bool ONE>
 __global__ void __launch_bounds__(kShadeBlock)
 KEscape(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, const __grid_constant__ PtJobDev one)
