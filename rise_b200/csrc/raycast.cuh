@@ -177,11 +177,13 @@ __device__ __forceinline__ void LoadVertices(const GpuTri* tris, int slot, float
 
 // ---- node decoders --------------------------------------------------------
 
-// A node's hit children: c[i] the link of child i, key[i] its entry distance
-// as ordered float bits with the child's number in the two low bits, or kMiss.
-// Distances from -0 up sort as integers; the two bits cost four ulps of an
-// ordering heuristic and make every key distinct.
+// A node's children: c[i] the link of child i (kEmpty when EXACT and missed),
+// key[i] its entry distance as float bits.  EXACT (closest hit): all the bits, and
+// those of +inf for a miss.  Otherwise (any hit, whose answer no order changes):
+// bits with the child's number in the two low ones, so that keys order as
+// integers from -0 up and are all distinct, and kMiss for a miss.
 constexpr int kMiss = INT_MAX;
+constexpr int kInfBits = 0x7f800000;
 struct ChildHits {
     int key[4];
     int c[4];
@@ -211,24 +213,34 @@ __device__ __forceinline__ float Min3(float a, float b, float c)
 //
 // The walk is bound by instruction issue (75 % of the issue slots, 14 of 32
 // lanes active), so the work of a visit is counted in instructions: products
-// run two to an instruction, and the four distances are ordered as integers
-// that carry the child's number (ten min / max, where ordering distance and
-// link pairs took five compares and twenty selects).  With the mixed
-// subtraction and the triangle rows (GpuTri): 4,194,304 incoherent closest-hit
-// rays on a 1M-triangle soup 3815 -> 3334 us over binary16 boxes, 3912 -> 3539
-// over 8-bit and 4542 -> 4402 over FP32 ones, which are bound by L1 instead.
+// run two to an instruction.  With the mixed subtraction and the triangle rows
+// (GpuTri), and the loads and the stack below: 4,194,304 incoherent closest-hit
+// rays on a 1M-triangle soup 3810 -> 2991 us over binary16 boxes, 3909 -> 3139
+// over 8-bit and 4527 -> 4140 over FP32 ones, which are bound by L1 instead.
+template <bool EXACT>
+__device__ __forceinline__ int HitKey(float tn, bool hit, int i, int& link)
+{
+    if (EXACT) {
+        link = hit ? link : kEmpty;
+        return hit ? __float_as_int(tn) : kInfBits;
+    }
+    return hit ? ((__float_as_int(tn) & ~3) | i) : kMiss;
+}
+
+template <bool EXACT>
 __device__ __forceinline__ int SlabKey(float nx, float ny, float nz, float fx, float fy, float fz, const RayPre& p,
-                                       float best, int i, bool present)
+                                       float best, int i, bool present, int& link)
 {
     const float2 ixy = make_float2(p.inv[0], p.inv[1]), izz = make_float2(p.inv[2], p.inv[2]);
     const float2 n = __fmul2_rn(make_float2(nx, ny), ixy), f = __fmul2_rn(make_float2(fx, fy), ixy);
     const float2 z = __fmul2_rn(make_float2(nz, fz), izz);
     const float tn = Max3(n.x, n.y, fmaxf(z.x, p.tmin));
     const float tf = Min3(f.x, f.y, fminf(z.y, best));
-    return tn <= tf && present ? ((__float_as_int(tn) & ~3) | i) : kMiss;
+    return HitKey<EXACT>(tn, tn <= tf && present, i, link);
 }
 
 // FP32 node: the low and high planes of an axis come in one load.
+template <bool EXACT>
 __device__ __forceinline__ void SlabF32(const GpuNode4* nodes, int ni, const RayPre& p, float best, ChildHits& h)
 {
     const float* base = reinterpret_cast<const float*>(nodes + ni);
@@ -247,10 +259,10 @@ __device__ __forceinline__ void SlabF32(const GpuNode4* nodes, int ni, const Ray
     h.c[0] = child.x; h.c[1] = child.y; h.c[2] = child.z; h.c[3] = child.w;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        h.key[i] = SlabKey((gx ? hxa[i] : lxa[i]) - p.o[0], (gy ? hya[i] : lya[i]) - p.o[1],
-                           (gz ? hza[i] : lza[i]) - p.o[2], (gx ? lxa[i] : hxa[i]) - p.o[0],
-                           (gy ? lya[i] : hya[i]) - p.o[1], (gz ? lza[i] : hza[i]) - p.o[2], p, best, i,
-                           h.c[i] != kEmpty);
+        h.key[i] = SlabKey<EXACT>((gx ? hxa[i] : lxa[i]) - p.o[0], (gy ? hya[i] : lya[i]) - p.o[1],
+                                  (gz ? hza[i] : lza[i]) - p.o[2], (gx ? lxa[i] : hxa[i]) - p.o[0],
+                                  (gy ? lya[i] : hya[i]) - p.o[1], (gz ? lza[i] : hza[i]) - p.o[2], p, best, i,
+                                  h.c[i] != kEmpty, h.c[i]);
 }
 
 // An 8-bit integer of a packed word as a float, exactly, without the
@@ -261,6 +273,7 @@ __device__ __forceinline__ float ByteMagic(unsigned w, int i)
 }
 
 // Quantised node: child slabs from 8-bit bounds, t = q * (2^e / d) + (origin - o) / d.
+template <bool EXACT>
 __device__ __forceinline__ void SlabQ8(const QNode4* nodes, int ni, const RayPre& p, float best, ChildHits& h)
 {
     const int4* base = reinterpret_cast<const int4*>(nodes + ni);
@@ -299,7 +312,7 @@ __device__ __forceinline__ void SlabQ8(const QNode4* nodes, int ni, const RayPre
         const float2 z = __ffma2_rn(__fadd2_rn(make_float2(ByteMagic(qn[2], i), ByteMagic(qf[2], i)), bias), szz, azz);
         const float tn = Max3(n.x, n.y, fmaxf(z.x, p.tmin));
         const float tf = Min3(f.x, f.y, fminf(z.y, best));
-        h.key[i] = tn <= tf && cnt[i] >= 0 ? ((__float_as_int(tn) & ~3) | i) : kMiss;
+        h.key[i] = HitKey<EXACT>(tn, tn <= tf && cnt[i] >= 0, i, h.c[i]);
     }
 }
 
@@ -315,6 +328,7 @@ __device__ __forceinline__ float HalfMinus(unsigned w, int hi, float o)
 
 // Half-precision node: the FP32 slab test on child boxes widened to binary16
 // (outward), planes picked by the direction's sign as in SlabKey.
+template <bool EXACT>
 __device__ __forceinline__ void SlabF16(const HNode4* nodes, int ni, const RayPre& p, float best, ChildHits& h)
 {
     const int4* base = reinterpret_cast<const int4*>(nodes + ni);
@@ -339,10 +353,10 @@ __device__ __forceinline__ void SlabF16(const HNode4* nodes, int ni, const RayPr
     h.c[0] = w3.x; h.c[1] = w3.y; h.c[2] = w3.z; h.c[3] = w3.w;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        h.key[i] = SlabKey(HalfMinus(n[0][i >> 1], i & 1, p.o[0]), HalfMinus(n[1][i >> 1], i & 1, p.o[1]),
-                           HalfMinus(n[2][i >> 1], i & 1, p.o[2]), HalfMinus(f[0][i >> 1], i & 1, p.o[0]),
-                           HalfMinus(f[1][i >> 1], i & 1, p.o[1]), HalfMinus(f[2][i >> 1], i & 1, p.o[2]), p, best, i,
-                           h.c[i] != kEmpty);
+        h.key[i] = SlabKey<EXACT>(HalfMinus(n[0][i >> 1], i & 1, p.o[0]), HalfMinus(n[1][i >> 1], i & 1, p.o[1]),
+                                  HalfMinus(n[2][i >> 1], i & 1, p.o[2]), HalfMinus(f[0][i >> 1], i & 1, p.o[0]),
+                                  HalfMinus(f[1][i >> 1], i & 1, p.o[1]), HalfMinus(f[2][i >> 1], i & 1, p.o[2]), p,
+                                  best, i, h.c[i] != kEmpty, h.c[i]);
 }
 
 // Child c of a node alone: its key and, in `link`, its link.  The same
@@ -353,19 +367,19 @@ __device__ __forceinline__ int ChildF32(const GpuNode4* nodes, int ni, int c, co
     const float* base = reinterpret_cast<const float*>(nodes + ni) + c;
     const int nx = p.inv[0] < 0.0f ? 4 : 0, ny = p.inv[1] < 0.0f ? 12 : 8, nz = p.inv[2] < 0.0f ? 20 : 16;
     link = __float_as_int(__ldg(base + 24));
-    return SlabKey(__ldg(base + nx) - p.o[0], __ldg(base + ny) - p.o[1], __ldg(base + nz) - p.o[2],
-                   __ldg(base + (4 - nx)) - p.o[0], __ldg(base + (20 - ny)) - p.o[1],
-                   __ldg(base + (36 - nz)) - p.o[2], p, best, c, link != kEmpty);
+    return SlabKey<false>(__ldg(base + nx) - p.o[0], __ldg(base + ny) - p.o[1], __ldg(base + nz) - p.o[2],
+                          __ldg(base + (4 - nx)) - p.o[0], __ldg(base + (20 - ny)) - p.o[1],
+                          __ldg(base + (36 - nz)) - p.o[2], p, best, c, link != kEmpty, link);
 }
 __device__ __forceinline__ int ChildF16(const HNode4* nodes, int ni, int c, const RayPre& p, float best, int& link)
 {
     const unsigned short* base = reinterpret_cast<const unsigned short*>(nodes + ni) + c;
     const int nx = p.inv[0] < 0.0f ? 12 : 0, ny = p.inv[1] < 0.0f ? 16 : 4, nz = p.inv[2] < 0.0f ? 20 : 8;
     link = __ldg(&nodes[ni].child[c]);
-    return SlabKey(HalfMinus(__ldg(base + nx), 0, p.o[0]), HalfMinus(__ldg(base + ny), 0, p.o[1]),
-                   HalfMinus(__ldg(base + nz), 0, p.o[2]), HalfMinus(__ldg(base + (12 - nx)), 0, p.o[0]),
-                   HalfMinus(__ldg(base + (20 - ny)), 0, p.o[1]), HalfMinus(__ldg(base + (28 - nz)), 0, p.o[2]), p, best,
-                   c, link != kEmpty);
+    return SlabKey<false>(HalfMinus(__ldg(base + nx), 0, p.o[0]), HalfMinus(__ldg(base + ny), 0, p.o[1]),
+                          HalfMinus(__ldg(base + nz), 0, p.o[2]), HalfMinus(__ldg(base + (12 - nx)), 0, p.o[0]),
+                          HalfMinus(__ldg(base + (20 - ny)), 0, p.o[1]), HalfMinus(__ldg(base + (28 - nz)), 0, p.o[2]),
+                          p, best, c, link != kEmpty, link);
 }
 __device__ __forceinline__ int ChildQ8(const QNode4* nodes, int ni, int c, const RayPre& p, float best, int& link)
 {
@@ -385,16 +399,17 @@ __device__ __forceinline__ int ChildQ8(const QNode4* nodes, int ni, int c, const
     link = __ldg(&n->child[c]);
     const float tn = Max3(tl[0], tl[1], fmaxf(tl[2], p.tmin));
     const float tf = Min3(th[0], th[1], fminf(th[2], best));
-    return tn <= tf && __ldg(&n->count[c]) >= 0 ? ((__float_as_int(tn) & ~3) | c) : kMiss;
+    return HitKey<false>(tn, tn <= tf && __ldg(&n->count[c]) >= 0, c, link);
 }
 
 template <class NodeT>
 struct Slab;
 template <>
 struct Slab<GpuNode4> {
+    template <bool EXACT>
     __device__ __forceinline__ static void Run(const GpuNode4* n, int i, const RayPre& p, float b, ChildHits& h)
     {
-        SlabF32(n, i, p, b, h);
+        SlabF32<EXACT>(n, i, p, b, h);
     }
     __device__ __forceinline__ static int One(const GpuNode4* n, int i, int c, const RayPre& p, float b, int& link)
     {
@@ -403,9 +418,10 @@ struct Slab<GpuNode4> {
 };
 template <>
 struct Slab<QNode4> {
+    template <bool EXACT>
     __device__ __forceinline__ static void Run(const QNode4* n, int i, const RayPre& p, float b, ChildHits& h)
     {
-        SlabQ8(n, i, p, b, h);
+        SlabQ8<EXACT>(n, i, p, b, h);
     }
     __device__ __forceinline__ static int One(const QNode4* n, int i, int c, const RayPre& p, float b, int& link)
     {
@@ -414,9 +430,10 @@ struct Slab<QNode4> {
 };
 template <>
 struct Slab<HNode4> {
+    template <bool EXACT>
     __device__ __forceinline__ static void Run(const HNode4* n, int i, const RayPre& p, float b, ChildHits& h)
     {
-        SlabF16(n, i, p, b, h);
+        SlabF16<EXACT>(n, i, p, b, h);
     }
     __device__ __forceinline__ static int One(const HNode4* n, int i, int c, const RayPre& p, float b, int& link)
     {
@@ -436,6 +453,50 @@ __device__ __forceinline__ int Child(const ChildHits& h, int key)
 {
     const int lo = (key & 1) ? h.c[1] : h.c[0], hi = (key & 1) ? h.c[3] : h.c[2];
     return (key & 2) ? hi : lo;
+}
+
+// After the call (ta, ca) holds the nearer entry; equal ones stay.
+__device__ __forceinline__ void CSwap(float& ta, int& ca, float& tb, int& cb)
+{
+    const bool sw = tb < ta;
+    const float t = sw ? tb : ta;
+    const int c = sw ? cb : ca;
+    tb = sw ? ta : tb;
+    cb = sw ? ca : cb;
+    ta = t;
+    ca = c;
+}
+
+// The children nearest first: with EXACT their links (kEmpty after the last hit
+// one), else their keys (kMiss).  The closest-hit walk keeps the first of
+// several triangles at one distance, so its order is part of its answer: by the
+// whole entry distances, with children at equal ones (coincident meshes have
+// the same boxes) in the order in which this network leaves them.  Keys that
+// gave two bits to the child's number turned 65,252 of 287,982 hits on three
+// coincident meshes to another of the three, and were no faster: decoding the
+// links took what the shorter sort gave (4,194,304 rays as above: binary16 3122
+// and 2991 us, 8-bit 3247 and 3139, FP32 4137 and 4140).  Any hit needs no such
+// order, and its keys sort in ten min / max.
+template <bool EXACT>
+__device__ __forceinline__ void Order(const ChildHits& h, int& k0, int& k1, int& k2, int& k3)
+{
+    if (EXACT) {
+        float t0 = __int_as_float(h.key[0]), t1 = __int_as_float(h.key[1]);
+        float t2 = __int_as_float(h.key[2]), t3 = __int_as_float(h.key[3]);
+        k0 = h.c[0]; k1 = h.c[1]; k2 = h.c[2]; k3 = h.c[3];
+        CSwap(t0, k0, t1, k1);
+        CSwap(t2, k2, t3, k3);
+        CSwap(t0, k0, t2, k2);
+        CSwap(t1, k1, t3, k3);
+        CSwap(t1, k1, t2, k2);
+        return;
+    }
+    k0 = h.key[0]; k1 = h.key[1]; k2 = h.key[2]; k3 = h.key[3];
+    CSwap(k0, k1);
+    CSwap(k2, k3);
+    CSwap(k0, k2);
+    CSwap(k1, k3);
+    CSwap(k1, k2);
 }
 
 // Per-lane traversal state of one ray.
@@ -539,40 +600,38 @@ __device__ __forceinline__ bool TraceRound(TraceState& s, const NodeT* __restric
         }
         if (s.node < 0) break;
         ChildHits h;
-        Slab<NodeT>::Run(nodes, s.node, s.p, s.best, h);
+        Slab<NodeT>::template Run<!ANY>(nodes, s.node, s.p, s.best, h);
         // The nearest hit child becomes the next node; the others are pushed
         // far to near (pushing them unsorted saved instructions and cost 11 %
         // in visits).
-        int k0 = h.key[0], k1 = h.key[1], k2 = h.key[2], k3 = h.key[3];
-        CSwap(k0, k1);
-        CSwap(k2, k3);
-        CSwap(k0, k2);
-        CSwap(k1, k3);
-        CSwap(k1, k2);
+        constexpr int kNone = ANY ? kMiss : kEmpty;
+        const auto link = [&](int k) { return ANY ? Child(h, k) : k; };
+        int k0, k1, k2, k3;
+        Order<!ANY>(h, k0, k1, k2, k3);
         if (!SPILL) {
             // One test for all three: the rows go on past the bound.
             if (s.sp > stk.bottom + kTraceStack * kStackStep) {
                 atomicOr(err, kErrStackOverflow);
-                k1 = k2 = k3 = kMiss;
+                k1 = k2 = k3 = kNone;
             }
-            if (k3 != kMiss) {
-                StoreShared(s.sp, Child(h, k3));
+            if (k3 != kNone) {
+                StoreShared(s.sp, link(k3));
                 s.sp += kStackStep;
             }
-            if (k2 != kMiss) {
-                StoreShared(s.sp, Child(h, k2));
+            if (k2 != kNone) {
+                StoreShared(s.sp, link(k2));
                 s.sp += kStackStep;
             }
-            if (k1 != kMiss) {
-                StoreShared(s.sp, Child(h, k1));
+            if (k1 != kNone) {
+                StoreShared(s.sp, link(k1));
                 s.sp += kStackStep;
             }
         } else {
-            if (k3 != kMiss) Push(s, stk, Child(h, k3), err);
-            if (k2 != kMiss) Push(s, stk, Child(h, k2), err);
-            if (k1 != kMiss) Push(s, stk, Child(h, k1), err);
+            if (k3 != kNone) Push(s, stk, link(k3), err);
+            if (k2 != kNone) Push(s, stk, link(k2), err);
+            if (k1 != kNone) Push(s, stk, link(k1), err);
         }
-        s.node = (k0 != kMiss) ? Child(h, k0) : Pop<SPILL>(s, stk);
+        s.node = (k0 != kNone) ? link(k0) : Pop<SPILL>(s, stk);
         // Postpone the first leaf met; keep descending until most lanes have one.
         if (s.node < 0 && s.node != kEmpty && s.leaf == kEmpty) {
             s.leaf = s.node;
