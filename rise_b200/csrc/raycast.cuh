@@ -113,11 +113,21 @@ __device__ __forceinline__ void PermutedOrigin(const RayPre& p, float& ox, float
     oz = p.rz == 0 ? p.o[0] : (p.rz == 16 ? p.o[1] : p.o[2]);
 }
 
-// Watertight ray/triangle test.  Returns true for a hit with tmin < t < tmax
-// and writes t and the barycentrics (alpha, beta) of v1 and v2, the
-// reference's (a, b) convention.  (ox, oy, oz) is PermutedOrigin.
+// A candidate hit: t = num / den (den > 0) and the quotient rounded, with the
+// barycentrics (alpha, beta) of v1 and v2, the reference's (a, b) convention.
+struct TriHit {
+    float num, den;
+    float t, a, b;
+};
+
+// A hit is nearer than tmax when its products say so: the rounded quotients of
+// two triangles can be equal where these are not.
+__device__ __forceinline__ bool Nearer(const TriHit& h, float tmax) { return !(h.num >= tmax * h.den); }
+
+// Watertight ray/triangle test.  Returns true for a hit with tmin < t < tmax.
+// (ox, oy, oz) is PermutedOrigin.
 __device__ __forceinline__ bool Watertight(const RayPre& p, const TriRows& r, float ox, float oy, float oz, float tmax,
-                                           float& tOut, float& aOut, float& bOut)
+                                           TriHit& h)
 {
     const float Az = r.z.x - oz, Bz = r.z.y - oz, Cz = r.z.z - oz;
     const float Ax = (r.x.x - ox) - p.sx * Az, Ay = (r.y.x - oy) - p.sy * Az;
@@ -141,12 +151,13 @@ __device__ __forceinline__ bool Watertight(const RayPre& p, const TriRows& r, fl
     // also drops triangles with edges below ~1e-6.
     if (!(adet >= 1e-12f * fabsf(p.sz))) return false;
     const float T = U * (p.sz * Az) + V * (p.sz * Bz) + W * (p.sz * Cz);
-    const float sT = copysignf(1.0f, det) * T;
-    if (sT <= p.tmin * adet || sT >= tmax * adet) return false;
+    h.num = copysignf(1.0f, det) * T;
+    h.den = adet;
+    if (h.num <= p.tmin * h.den || !Nearer(h, tmax)) return false;
     const float rcp = 1.0f / det;
-    tOut = T * rcp;
-    aOut = V * rcp;
-    bOut = W * rcp;
+    h.t = T * rcp;
+    h.a = V * rcp;
+    h.b = W * rcp;
     return true;
 }
 
@@ -361,26 +372,29 @@ __device__ __forceinline__ void SlabF16(const HNode4* nodes, int ni, const RayPr
 
 // Child c of a node alone: its key and, in `link`, its link.  The same
 // arithmetic as the whole node's, for walks that give a child to each lane.
+template <bool EXACT>
 __device__ __forceinline__ int ChildF32(const GpuNode4* nodes, int ni, int c, const RayPre& p, float best, int& link)
 {
     // Float offsets of lox, hix, loy, hiy, loz, hiz: 0, 4, 8, 12, 16, 20.
     const float* base = reinterpret_cast<const float*>(nodes + ni) + c;
     const int nx = p.inv[0] < 0.0f ? 4 : 0, ny = p.inv[1] < 0.0f ? 12 : 8, nz = p.inv[2] < 0.0f ? 20 : 16;
     link = __float_as_int(__ldg(base + 24));
-    return SlabKey<false>(__ldg(base + nx) - p.o[0], __ldg(base + ny) - p.o[1], __ldg(base + nz) - p.o[2],
+    return SlabKey<EXACT>(__ldg(base + nx) - p.o[0], __ldg(base + ny) - p.o[1], __ldg(base + nz) - p.o[2],
                           __ldg(base + (4 - nx)) - p.o[0], __ldg(base + (20 - ny)) - p.o[1],
                           __ldg(base + (36 - nz)) - p.o[2], p, best, c, link != kEmpty, link);
 }
+template <bool EXACT>
 __device__ __forceinline__ int ChildF16(const HNode4* nodes, int ni, int c, const RayPre& p, float best, int& link)
 {
     const unsigned short* base = reinterpret_cast<const unsigned short*>(nodes + ni) + c;
     const int nx = p.inv[0] < 0.0f ? 12 : 0, ny = p.inv[1] < 0.0f ? 16 : 4, nz = p.inv[2] < 0.0f ? 20 : 8;
     link = __ldg(&nodes[ni].child[c]);
-    return SlabKey<false>(HalfMinus(__ldg(base + nx), 0, p.o[0]), HalfMinus(__ldg(base + ny), 0, p.o[1]),
+    return SlabKey<EXACT>(HalfMinus(__ldg(base + nx), 0, p.o[0]), HalfMinus(__ldg(base + ny), 0, p.o[1]),
                           HalfMinus(__ldg(base + nz), 0, p.o[2]), HalfMinus(__ldg(base + (12 - nx)), 0, p.o[0]),
                           HalfMinus(__ldg(base + (20 - ny)), 0, p.o[1]), HalfMinus(__ldg(base + (28 - nz)), 0, p.o[2]),
                           p, best, c, link != kEmpty, link);
 }
+template <bool EXACT>
 __device__ __forceinline__ int ChildQ8(const QNode4* nodes, int ni, int c, const RayPre& p, float best, int& link)
 {
     const QNode4* n = nodes + ni;
@@ -399,7 +413,7 @@ __device__ __forceinline__ int ChildQ8(const QNode4* nodes, int ni, int c, const
     link = __ldg(&n->child[c]);
     const float tn = Max3(tl[0], tl[1], fmaxf(tl[2], p.tmin));
     const float tf = Min3(th[0], th[1], fminf(th[2], best));
-    return HitKey<false>(tn, tn <= tf && __ldg(&n->count[c]) >= 0, c, link);
+    return HitKey<EXACT>(tn, tn <= tf && __ldg(&n->count[c]) >= 0, c, link);
 }
 
 template <class NodeT>
@@ -411,9 +425,10 @@ struct Slab<GpuNode4> {
     {
         SlabF32<EXACT>(n, i, p, b, h);
     }
+    template <bool EXACT>
     __device__ __forceinline__ static int One(const GpuNode4* n, int i, int c, const RayPre& p, float b, int& link)
     {
-        return ChildF32(n, i, c, p, b, link);
+        return ChildF32<EXACT>(n, i, c, p, b, link);
     }
 };
 template <>
@@ -423,9 +438,10 @@ struct Slab<QNode4> {
     {
         SlabQ8<EXACT>(n, i, p, b, h);
     }
+    template <bool EXACT>
     __device__ __forceinline__ static int One(const QNode4* n, int i, int c, const RayPre& p, float b, int& link)
     {
-        return ChildQ8(n, i, c, p, b, link);
+        return ChildQ8<EXACT>(n, i, c, p, b, link);
     }
 };
 template <>
@@ -435,9 +451,10 @@ struct Slab<HNode4> {
     {
         SlabF16<EXACT>(n, i, p, b, h);
     }
+    template <bool EXACT>
     __device__ __forceinline__ static int One(const HNode4* n, int i, int c, const RayPre& p, float b, int& link)
     {
-        return ChildF16(n, i, c, p, b, link);
+        return ChildF16<EXACT>(n, i, c, p, b, link);
     }
 };
 
@@ -646,18 +663,18 @@ __device__ __forceinline__ bool TraceRound(TraceState& s, const NodeT* __restric
     PermutedOrigin(s.p, ox, oy, oz);
     while (slot >= 0) {
         const TriRows r = LoadRows(tris, slot, s.p);
-        float t, a, b;
-        if (Watertight(s.p, r, ox, oy, oz, s.best, t, a, b)) {
+        TriHit hit;
+        if (Watertight(s.p, r, ox, oy, oz, s.best, hit)) {
             if (ANY) {
                 s.bestSlot = slot;
                 s.node = kEmpty;
                 s.leaf = kEmpty;
                 return true;
             }
-            s.best = t;
+            s.best = hit.t;
             s.bestSlot = slot;
-            s.ba = a;
-            s.bb = b;
+            s.ba = hit.a;
+            s.bb = hit.b;
         }
         // The last triangle of a leaf is flagged; the array bound is a second
         // stop so a leaf walk never leaves the buffer.
@@ -685,10 +702,17 @@ __device__ __forceinline__ bool TraceRound(TraceState& s, const NodeT* __restric
 // node.  One step does the work of up to eight dependent steps of the lane
 // walk, so a small batch, and the end of a large one, waits for memory a few
 // times instead of once per node and triangle (1,000 rays on a 100k-triangle
-// soup: 109 -> 21 us).  The walk tests boxes in
-// another order and with the group's best distance, and finds the same
-// closest triangle (of several at exactly the same distance, the one that
-// comes first in leaf order among those a step tests).
+// soup: 109 -> 21 us).
+//
+// A closest hit is the lane walk's, triangle for triangle: which walk ends a ray
+// depends on its neighbours and on timing, and must not show where triangles lie
+// at one distance.  So children are ordered by the lane walk's Order, a leaf
+// waits on the stack until all nodes before it have been opened, and the hits of
+// a step are taken in the lane walk's order with its comparison.  Only boxes are
+// tested early, with a best distance that is at most too large.  Testing leaves
+// as they came gave other triangles for 1,266 of 600,000 rays on a soup whose
+// triangles lie there twice, 535 of them from run to run; the order costs 20,000
+// rays on a 300k-triangle soup 99 -> 113 us and 100,003 nothing (178 us).
 //
 // Everything lives in the warp's part of the stack memory: with D the deepest
 // lane stack, rows D + 1 .. D + m keep the state of the m rays, a row each,
@@ -703,13 +727,6 @@ enum CoopWord : int {
     kCoO = 0, kCoInv = 3, kCoTmin = 6, kCoRows = 7, kCoS = 8, kCoBest = 11, kCoSlot = 12, kCoA = 13, kCoB = 14,
     kCoNode = 15, kCoLeaf = 16, kCoSp = 17, kCoLane = 18, kCoNodes = 19, kCoTris = 21, kCoNtri = 23
 };
-
-// Orders floats as integers.
-__device__ __forceinline__ int OrderedBits(float t)
-{
-    const int i = __float_as_int(t);
-    return i ^ ((i >> 31) & 0x7fffffff);
-}
 
 // Whether a warp whose lanes with `live` set still hold a ray should finish
 // them together: few rays, and room above the lane stacks for their state
@@ -752,7 +769,6 @@ __device__ __forceinline__ void CoopWalk(int* rows, int D, int m, unsigned* err)
         p.sy = __int_as_float(word(row, kCoS + 1));
         p.sz = __int_as_float(word(row, kCoS + 2));
         float best = __int_as_float(word(row, kCoBest));
-        int bestSlot = word(row, kCoSlot);
         const NodeT* nd = reinterpret_cast<const NodeT*>(((unsigned long long)(unsigned)word(row, kCoNodes + 1) << 32) |
                                                          (unsigned)word(row, kCoNodes));
         const GpuTri* tr = reinterpret_cast<const GpuTri*>(((unsigned long long)(unsigned)word(row, kCoTris + 1) << 32) |
@@ -778,40 +794,40 @@ __device__ __forceinline__ void CoopWalk(int* rows, int D, int m, unsigned* err)
             // Eight entries at once while that leaves a depth-first walk of one
             // entry's subtree (at most kBound more) room above them.
             const int take = max(1, min(min(8, sp), (cap - kBound - sp) / 3));
-            // Group `take - 1` holds the top entry, so its children end up on top.
-            const int e = (int)group < take ? entry(sp - take + (int)group) : kEmpty;
+            // Group 0 holds the top entry: lanes are in the order of the lane walk.
+            const int e = (int)group < take ? entry(sp - 1 - (int)group) : kEmpty;
             sp -= take;
             __syncwarp();
-            int key = kMiss, link = kEmpty;
-            if (e >= 0) key = Slab<NodeT>::One(nd, e, (int)c, p, best, link);
-            bool hit = false;
-            float t = 0.0f, al = 0.0f, be = 0.0f;
-            int at = (e < 0 && e != kEmpty) ? ~e + (int)c : -1, hitSlot = -1;
-            while (__any_sync(kFull, at >= 0)) {
-                bool last = false, tested = false;
-                float tt, ta, tb;
-                if (at >= 0) {
-                    const TriRows r = LoadRows(tr, min(at, nt - 1), p);
-                    last = __float_as_int(r.x.w) < 0 || at >= nt - 1;
-                    tested = Watertight(p, r, ox, oy, oz, best, tt, ta, tb);
-                }
-                // Lanes past the leaf's last triangle looked at another leaf's.
-                const unsigned lasts = (__ballot_sync(kFull, last) >> (group * 4u)) & 0xfu;
-                if (tested && !(lasts & ((1u << c) - 1u)) && (hitSlot < 0 || tt < t)) {
-                    hit = true;
-                    t = tt; al = ta; be = tb;
-                    hitSlot = at;
-                }
-                at = at >= 0 && !lasts ? at + 4 : -1;
+            const unsigned ahead = (1u << (group * 4u)) - 1u;   // lanes of the groups before this one
+            const unsigned nodes = __ballot_sync(kFull, e >= 0);
+            int key = ANY ? kMiss : kInfBits, link = kEmpty;
+            if (e >= 0) key = Slab<NodeT>::template One<!ANY>(nd, e, (int)c, p, best, link);
+            if (ANY && key == kMiss) link = kEmpty;
+            // Four triangles of a leaf, a lane each; a longer one goes back with
+            // the rest, and leaves after it wait as they do for a node.
+            const bool leaf = e < 0 && e != kEmpty;
+            bool open = leaf && (ANY || !(nodes & ahead));
+            const int at = leaf ? ~e + (int)c : -1;
+            bool last = false, tested = false;
+            TriHit h{0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            if (open) {
+                const TriRows r = LoadRows(tr, min(at, nt - 1), p);
+                last = __float_as_int(r.x.w) < 0 || at >= nt - 1;
+                tested = Watertight(p, r, ox, oy, oz, best, h);
             }
-            if (__any_sync(kFull, hit)) {
-                const int ord = hit ? OrderedBits(t) : INT_MAX;
-                const int lo = __reduce_min_sync(kFull, ord);
-                const int slot = __reduce_min_sync(kFull, hit && ord == lo ? hitSlot : INT_MAX);
-                const int from = __ffs(__ballot_sync(kFull, hit && ord == lo && hitSlot == slot)) - 1;
-                best = __shfl_sync(kFull, t, from);
-                bestSlot = slot;
-                const float ba = __shfl_sync(kFull, al, from), bb = __shfl_sync(kFull, be, from);
+            const unsigned lasts = (__ballot_sync(kFull, last) >> (group * 4u)) & 0xfu;
+            const bool more = open && !lasts;
+            const unsigned unfinished = __ballot_sync(kFull, more);
+            if (!ANY && (unfinished & ahead)) open = false;
+            // Lanes past the leaf's last triangle looked at another leaf's.
+            tested = tested && open && !(lasts & ((1u << c) - 1u));
+            unsigned cand = __ballot_sync(kFull, tested);
+            const bool found = cand != 0u;
+            while (cand) {
+                const int from = __ffs(cand) - 1;
+                best = __shfl_sync(kFull, h.t, from);
+                const int slot = __shfl_sync(kFull, at, from);
+                const float ba = __shfl_sync(kFull, h.a, from), bb = __shfl_sync(kFull, h.b, from);
                 if (lane == 0) {
                     word(row, kCoBest) = __float_as_int(best);
                     word(row, kCoSlot) = slot;
@@ -819,18 +835,43 @@ __device__ __forceinline__ void CoopWalk(int* rows, int D, int m, unsigned* err)
                     word(row, kCoB) = __float_as_int(bb);
                 }
                 if (ANY) break;
+                cand = __ballot_sync(kFull, tested && (int)lane > from && Nearer(h, best));
             }
-            // Push the hit children: a lower group's below a higher group's,
-            // within a group the farther ones first.
-            const unsigned hits = __ballot_sync(kFull, key != kMiss);
+            if (ANY && found) break;
+            if (leaf && c == 0u && (!open || more)) {
+                key = 0;
+                link = open ? e - 4 : e;   // ~(first + 4)
+            }
+            // Push: a group's entries above a later group's, within a group the
+            // farther ones first.
+            const unsigned hits = __ballot_sync(kFull, link != kEmpty);
             int rank = 0;
+            bool equal = false;
 #pragma unroll
-            for (int x = 1; x < 4; ++x) {
+            for (unsigned x = 1; x < 4; ++x) {
                 const int other = __shfl_xor_sync(kFull, key, x);
-                rank += other != kMiss && other > key;
+                if (ANY) {
+                    rank += other != kMiss && other > key;
+                } else {
+                    rank += ((hits >> (lane ^ x)) & 1u) && __int_as_float(other) > __int_as_float(key);
+                    equal |= __int_as_float(other) == __int_as_float(key);
+                }
             }
-            const int pos = sp + __popc(hits & ((1u << (group * 4u)) - 1u)) + rank;
-            if (key != kMiss) {
+            if (!ANY && __any_sync(kFull, equal && link != kEmpty)) {
+                // Children at one distance: the order is the network's.
+                ChildHits ch;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    ch.key[j] = __shfl_sync(kFull, key, (int)(lane & ~3u) + j);
+                    ch.c[j] = (hits >> ((lane & ~3u) + j)) & 1u ? j : kEmpty;
+                }
+                int k0, k1, k2, k3;
+                Order<true>(ch, k0, k1, k2, k3);
+                const int me = (int)c;
+                rank = (k3 != kEmpty && me != k3) + (k2 != kEmpty && me != k3 && me != k2) + (k1 != kEmpty && me == k0);
+            }
+            const int pos = sp + __popc((hits >> (group * 4u)) >> 4u) + rank;
+            if (link != kEmpty) {
                 if (pos < cap) entry(pos) = link;
                 else atomicOr(err, kErrStackOverflow);
             }
@@ -1036,13 +1077,13 @@ __device__ __forceinline__ bool TraceW8(W8State& s, const WNode8* __restrict__ n
             tg.y &= tg.y - 1u;
             const unsigned slot = tg.x + k;
             const TriRows r = LoadRows(tris, (int)slot, s.p);
-            float t, al, be;
-            if (Watertight(s.p, r, ox, oy, oz, s.best, t, al, be)) {
+            TriHit hit;
+            if (Watertight(s.p, r, ox, oy, oz, s.best, hit)) {
                 s.bestSlot = (int)slot;
                 if (ANY) return true;
-                s.best = t;
-                s.ba = al;
-                s.bb = be;
+                s.best = hit.t;
+                s.ba = hit.a;
+                s.bb = hit.b;
             }
         }
         if (!(s.ng.y & 0xff000000u)) {

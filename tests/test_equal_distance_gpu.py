@@ -11,7 +11,9 @@ Python gives the one right answer.
 import numpy as np
 import pytest
 
-from rise_b200 import raycaster
+from rise_b200 import raycaster, scenes
+
+from risemesh_io import risemesh_bytes, soup_mesh
 
 pytestmark = pytest.mark.gpu
 
@@ -117,4 +119,70 @@ def test_children_at_one_distance_keep_their_order(layout, planes):
         n = many_rays(ctx)
         got = cast(raycaster.RayCaster(s), np.tile(rays, (n // RAYS + 1, 1))[:n])["prim"]
         assert np.array_equal(got, np.tile(want, n // RAYS + 1)[:n])
+        s.close()
+
+
+def soup_twice():
+    tri = scenes.soup_triangles(10_000, seed=3)
+    return np.concatenate([tri, tri])[np.random.default_rng(7).permutation(20_000)], None
+
+
+def long_leaves():
+    """Leaves of twelve coincident triangles, in both windings."""
+    tri = scenes.soup_triangles(3_000, seed=3)
+    both = np.concatenate([tri, tri[:, [3, 4, 5, 0, 1, 2, 6, 7, 8]]] * 6)
+    return both[np.random.default_rng(7).permutation(len(both))], None
+
+
+def merged_meshes():
+    tri = scenes.soup_triangles(6_000, seed=3)
+    return None, [tri[:4000], tri[2000:], tri[1000:5000]]
+
+
+def deep_twice():
+    """A tree deeper than the shared-memory stack."""
+    tri = scenes.nested_clusters()
+    return np.concatenate([tri, tri]), None
+
+
+@pytest.mark.parametrize("make,layout", [
+    (m, v) for m in (soup_twice, long_leaves, merged_meshes, deep_twice) for v in ("f32", "q8", "f16", "w8")
+    if not (m is deep_twice and v == "w8")])   # the eight-wide layout refuses its leaves
+def test_coincident_triangles_answer_alike_in_every_batch(make, layout):
+    tri, parts = make()
+    with raycaster.Context(0) as ctx:
+        s = raycaster.Scene(ctx)
+        for p in parts or []:
+            nodes2, prims, _ = raycaster.build_host_bvh(p)
+            pts, idx = soup_mesh(p)
+            s.add_risemesh(raycaster.RiseMesh(risemesh_bytes(pts, idx, nodes2=nodes2, prims=prims)))
+        if tri is not None:
+            s.add_triangles(tri)
+        s.commit(layout)
+        rc = raycaster.RayCaster(s)
+        n = many_rays(ctx)
+        rays = scenes.cluster_rays(tri, n, 5) if make is deep_twice else scenes.sphere_rays(n, 5)
+        hits = cast(rc, rays)
+        assert (hits["prim"] >= 0).mean() > 0.05
+        for k in (1, 5, 64, 4095, 20_000, 100_003, n - 4097):
+            for repeat in range(10 if k > 20_000 else 2):
+                assert cast(rc, rays[:k]).tobytes() == hits[:k].tobytes(), (k, repeat)
+        s.close()
+
+
+@pytest.mark.parametrize("planes", PLANES)
+@pytest.mark.parametrize("layout", ["f32", "f16"])
+def test_small_batches_keep_the_first_triangle_met(layout, planes):
+    tri = right_triangles(400, planes, 3)
+    _, prims, nodes = raycaster.build_host_bvh(tri)
+    rays = upward_rays(RAYS, 4)
+    want = np.array([walk(tri, prims, nodes, r) for r in rays])
+    with raycaster.Context(0) as ctx:
+        s = raycaster.Scene(ctx)
+        s.add_triangles(tri)
+        s.commit(layout)
+        rc = raycaster.RayCaster(s)
+        for n in (1, 3, 64, RAYS):
+            for k in range(0, RAYS, max(n, 32)):
+                assert np.array_equal(cast(rc, rays[k:k + n])["prim"], want[k:k + n]), (n, k)
         s.close()
