@@ -557,8 +557,11 @@ int EngineRender(rtb200_engine* e, rtb200_job* const* jobs, const int32_t* spp, 
 // fewer and fuller iterations (200 x 150 at 16 spp 1.48 -> 1.32 ms, at 32 spp 2.48
 // -> 2.28; more than the request's paths, or than 2^19, was no faster there).
 // Not for requests that fold their film step by step: a larger pool would add
-// more samples in FP32 between folds.  And only in a context without a memory
-// budget that holds little, so that no later allocation misses the memory.
+// more samples in FP32 between folds.  Not for jobs with a progress callback
+// either: it stops a request by giving out no more samples, and a pool that
+// takes the whole request leaves none to keep back.  And only in a context
+// without a memory budget that holds little, so that no later allocation misses
+// the memory.
 constexpr size_t kRoomyBytes = size_t(16) << 30;
 
 int JobEngine(rtb200_job* j, int spp)
@@ -567,11 +570,11 @@ int JobEngine(rtb200_job* j, int spp)
     const int base = j->rs.max_paths > 0 ? j->rs.max_paths
                                          : (int)std::min<int64_t>(std::max<int64_t>((int64_t)j->npix * 8, 65536), 1 << 21);
     const long long paths = (long long)j->npix * spp * j->spectral;
-    const bool folds = spp >= kFoldEverySpp;
+    const bool keep_base = spp >= kFoldEverySpp || j->progress;
     const bool roomy = j->rs.max_paths <= 0 && !ctx->budget && ctx->in_use < kRoomyBytes;
-    const int want = roomy && !folds ? std::max(base, (int)std::min<long long>(paths, 1 << 19)) : base;
-    if (j->own && (folds ? j->own->capacity <= ((base + 31) & ~31) : j->own->capacity >= want)) return RTB200_OK;
-    if (j->own && folds) {
+    const int want = roomy && !keep_base ? std::max(base, (int)std::min<long long>(paths, 1 << 19)) : base;
+    if (j->own && (keep_base ? j->own->capacity <= ((base + 31) & ~31) : j->own->capacity >= want)) return RTB200_OK;
+    if (j->own && keep_base) {
         EngineDestroy(j->own);
         j->own = nullptr;
     }
