@@ -82,8 +82,14 @@ int rtb200_ctx_create(int device, size_t budget_bytes, rtb200_ctx** out);
 int rtb200_ctx_destroy(rtb200_ctx* ctx);
 /* Message for the last failing call on this context ("" if none). */
 const char* rtb200_last_error(const rtb200_ctx* ctx);
-/* Device bytes currently held by the context. */
+/* Device bytes held by the context's scenes, jobs, engines and calls.  Blocks
+ * kept for reuse after a job or engine is destroyed (its films and path pool) are
+ * not counted: at most 4 GB, freed when an allocation of the context or its
+ * budget needs them, by rtb200_ctx_trim and with the context. */
 size_t rtb200_ctx_bytes_in_use(const rtb200_ctx* ctx);
+/* Free the blocks kept for reuse, device and pinned host memory, for other users
+ * of the device.  Waits for the context's work. */
+int rtb200_ctx_trim(rtb200_ctx* ctx);
 
 /* ---- scenes ------------------------------------------------------------ */
 

@@ -29,6 +29,7 @@ SIGNATURES = {
     "rtb200_ctx_destroy": (ctypes.c_int, [_vp]),
     "rtb200_last_error": (ctypes.c_char_p, [_vp]),
     "rtb200_ctx_bytes_in_use": (ctypes.c_size_t, [_vp]),
+    "rtb200_ctx_trim": (ctypes.c_int, [_vp]),
     "rtb200_scene_create": (ctypes.c_int, [_vp, _pvp]),
     "rtb200_scene_add_mesh": (ctypes.c_int, [_vp, _vp, _i64, _vp, _i64, _i32, _i32]),
     "rtb200_scene_commit": (ctypes.c_int, [_vp, _i32]),

@@ -263,6 +263,17 @@ const char* rtb200_last_error(const rtb200_ctx* ctx) { return ctx ? ctx->err.c_s
 
 size_t rtb200_ctx_bytes_in_use(const rtb200_ctx* ctx) { return ctx ? ctx->in_use : 0; }
 
+int rtb200_ctx_trim(rtb200_ctx* ctx)
+{
+    if (!ctx) return RTB200_E_INVALID;
+    std::lock_guard<std::mutex> g(ctx->mu);
+    cudaSetDevice(ctx->device);
+    DevReleaseCache(ctx);
+    for (void* p : ctx->pinned) cudaFreeHost(p);
+    ctx->pinned.clear();
+    return CudaCheck(ctx, cudaStreamSynchronize(ctx->stream), "trim");
+}
+
 int rtb200_scene_create(rtb200_ctx* ctx, rtb200_scene** out)
 {
     if (!ctx || !out) return RTB200_E_INVALID;

@@ -42,7 +42,14 @@ class Context:
         self.device = device
 
     def bytes_in_use(self):
+        """Device bytes of live scenes, jobs and engines; blocks kept for reuse
+        (see trim) are not counted."""
         return lib().rtb200_ctx_bytes_in_use(self.h)
+
+    def trim(self):
+        """Free the memory of closed jobs and engines that is kept for the next
+        ones (at most 4 GB on the device)."""
+        check(lib().rtb200_ctx_trim(self.h), self.h)
 
     def close(self):
         if self.h:
