@@ -416,8 +416,12 @@ int EngineStep(rtb200_engine* e, int iterations, bool graph)
     if (e->h_cnt[kCntCount]) return SetError(ctx, RTB200_E_DEVICE, "device error word set (traversal stack overflow)");
     // Per-job statistics: attribute this step's segments to the active jobs
     // (the last iteration's are still in its queue counters).
-    const long long seg = (unsigned)e->h_cnt[kCntSegments] + (unsigned)e->h_cnt[kCntActive],
-                    sh = (unsigned)e->h_cnt[kCntShadowRays] + (unsigned)e->h_cnt[kCntShadow];
+    const auto total = [&](int sum, int last) {
+        unsigned long long v;
+        std::memcpy(&v, e->h_cnt + sum, sizeof(v));
+        return (long long)(v + (unsigned)e->h_cnt[last]);
+    };
+    const long long seg = total(kCntSegments, kCntActive), sh = total(kCntShadowRays, kCntShadow);
     const long long dseg = seg - e->seg_seen, dsh = sh - e->shadow_seen;
     e->seg_seen = seg;
     e->shadow_seen = sh;

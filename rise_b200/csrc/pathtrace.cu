@@ -323,8 +323,8 @@ KAssign(const PtJobDev* __restrict__ jobs, const int* __restrict__ ids, PtQueues
     if (threadIdx.x == 0) {
         int* cnt = Q.cnt;
         for (int c = 0; c < kShadeClasses; ++c) cnt[kCntClass + c] = 0;
-        cnt[kCntSegments] += cnt[kCntActive];
-        cnt[kCntShadowRays] += cnt[kCntShadow];
+        Counter64(cnt, kCntSegments) += (unsigned)cnt[kCntActive];
+        Counter64(cnt, kCntShadowRays) += (unsigned)cnt[kCntShadow];
         cnt[kCntActive] = cnt[kCntFreshRays] = cnt[kCntNext + (parity ^ 1)];
         cnt[kCntNext + parity] = 0;
         cnt[kCntFree] = n;

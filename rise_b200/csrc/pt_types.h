@@ -169,8 +169,6 @@ enum PtCounter : int {
     kCntFree = 2,       // finished / empty slots to regenerate
     kCntFreeNext = 3,
     kCntShadow = 4,
-    kCntSegments = 5,   // extended rays (statistics)
-    kCntShadowRays = 6,
     kCntAssigned = 7,   // free slots given camera samples this iteration
     kCntClass = 8,      // kCntClass + c: active paths of shading class c (KClassify)
     kCntJobs = 12,      // entries of the job id list (written by the host)
@@ -178,8 +176,14 @@ enum PtCounter : int {
     // p and read by the next one, whose KExtend may still read it while KAssign
     // prepares the counters of the iteration after.
     kCntNext = 14,
-    kCntCount = 16,
+    // Statistics of the iterations before this one, 64 bits each: a kept engine
+    // passes 2^32 shadow rays within seconds.
+    kCntSegments = 16,   // extended rays
+    kCntShadowRays = 18,
+    kCntCount = 20,
 };
+// A 64-bit counter at an even index of the counters.
+RTB_HD unsigned long long& Counter64(int* cnt, int k) { return *reinterpret_cast<unsigned long long*>(cnt + k); }
 
 struct PtEnvMap;   // env_map.h
 
