@@ -282,6 +282,7 @@ int rtb200_scene_create(rtb200_ctx* ctx, rtb200_scene** out)
     rtb200_scene* s = new (std::nothrow) rtb200_scene();
     if (!s) return SetError(ctx, RTB200_E_OOM, "host allocation failed");
     s->ctx = ctx;
+    s->id = ++ctx->scenes_made;
     cudaSetDevice(ctx->device);
     void* p = nullptr;
     int rc = DevAlloc(ctx, &p, 256);

@@ -31,10 +31,13 @@ struct rtb200_ctx {
     size_t cached = 0;
     // Pinned blocks of destroyed engines, all of one size (engine.cpp).
     std::vector<void*> pinned;
+    uint64_t scenes_made = 0;
 };
 
 struct rtb200_scene {
     rtb200_ctx* ctx = nullptr;
+    // The scene's number in its context.  Its address may be a destroyed scene's.
+    uint64_t id = 0;
     // host geometry, scene-wide triangle numbering
     std::vector<float> tri9;
     std::vector<int32_t> tri_material;

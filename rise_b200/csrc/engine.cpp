@@ -136,7 +136,7 @@ struct rtb200_engine {
     bool ggraph = false;                   // gexec holds a capture for the fields below
     int glayout = -1;
     bool gspill = false;
-    const rtb200_scene* gscene = nullptr;  // the shared scene, or null when jobs differ
+    uint64_t gscene = 0;                   // number of the shared scene, or 0 when jobs differ
     bool gclassify = false;
     bool genv_image = false;
     bool gcoop = false;
@@ -359,7 +359,9 @@ int EngineStep(rtb200_engine* e, int iterations, bool graph)
     PtLaunch L = MakeLaunch(e);
     cudaError_t err = cudaSuccess;
     if (graph) {
-        const rtb200_scene* us = L.uniform ? e->owner[e->active[0]]->scene : nullptr;
+        // By number: a capture holds the scene's pointers, and a scene made after
+        // another was destroyed can have its address.
+        const uint64_t us = L.uniform ? e->owner[e->active[0]]->scene->id : 0;
         if (!e->ggraph || e->glayout != L.layout || e->gspill != L.spill ||
             e->gscene != us || e->gclassify != L.classify || e->gshade_class != L.shade_class ||
             e->genv_image != L.env_image || e->gcoop != L.coop) {
