@@ -486,6 +486,12 @@ int rtb200_engine_retire(rtb200_engine* engine, rtb200_job* job);
  * reports done == total and the job can be retired (a served request that
  * is abandoned or cancelled by its client). */
 int rtb200_engine_cancel(rtb200_engine* engine, rtb200_job* job);
+/* Requests not yet retired are withdrawn: film, sample count and adaptive state
+ * of their jobs stay as before the request, and the jobs can be rendered again.
+ * A request whose job has already taken part of its samples (adaptive jobs,
+ * requests of 64 samples per pixel and more) ends as by rtb200_engine_cancel
+ * instead: the pixel samples started are finished and count.  Should that fail on
+ * the device, the job's calls return RTB200_E_DEVICE until it is destroyed. */
 int rtb200_engine_destroy(rtb200_engine* engine);
 /* Wavefront iterations rtb200_engine_render runs between host polls of the
  * jobs' progress (default 4; rounded up to even, 2 .. 1024).  Fewer polls

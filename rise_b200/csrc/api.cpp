@@ -290,6 +290,7 @@ int rtb200_scene_create(rtb200_ctx* ctx, rtb200_scene** out)
     cudaMemset(p, 0, 256);
     s->d_counter = (unsigned long long*)p;
     s->d_err = (unsigned*)((char*)p + 64);
+    ctx->scenes.insert(s->id);
     *out = s;
     return RTB200_OK;
 }
@@ -522,6 +523,7 @@ int rtb200_scene_destroy(rtb200_scene* s)
     DevFree(ctx, s->d_out, s->stage_out);
     DevFree(ctx, s->d_counter, 256);
     FreeShading(s);
+    ctx->scenes.erase(s->id);
     delete s;
     return RTB200_OK;
 }

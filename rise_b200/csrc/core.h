@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <mutex>
 #include <unordered_map>
+#include <unordered_set>
 #include <string>
 #include <vector>
 
@@ -31,7 +32,9 @@ struct rtb200_ctx {
     size_t cached = 0;
     // Pinned blocks of destroyed engines, all of one size (engine.cpp).
     std::vector<void*> pinned;
+    // Scenes made, and those that exist, by number.
     uint64_t scenes_made = 0;
+    std::unordered_set<uint64_t> scenes;
 };
 
 struct rtb200_scene {

@@ -70,6 +70,7 @@ size_t Align(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct rtb200_job {
     rtb200_scene* scene = nullptr;
+    uint64_t scene_id = 0;
     rtb200_render_settings rs{};
     PtCamera cam{};
     PtSettings set{};
@@ -104,6 +105,8 @@ struct rtb200_job {
     rtb200_engine* engine = nullptr;   // engine the job is submitted to
     int entry = -1;
     long long pending_spp = 0;
+    bool folded = false;               // part of the request in flight is in the film's sums
+    bool spoiled = false;              // samples of a failed request are in the film's sums
     rtb200_engine* own = nullptr;      // private engine of rtb200_job_render
 };
 
@@ -259,12 +262,51 @@ int EngineCreate(rtb200_ctx* ctx, int capacity, rtb200_engine** out)
     return RTB200_OK;
 }
 
+int EngineStep(rtb200_engine* e, int iterations, bool graph);
+int EngineRetire(rtb200_engine* e, rtb200_job* j);
+void CancelEntry(rtb200_engine* e, rtb200_job* j);
+bool JobDone(const rtb200_engine* e, int entry);
+
+// Ends what is still submitted.  Between requests a job's accumulator is clear
+// and its sums belong to its sample count; a request cut off anywhere would leave
+// samples behind that the next one counts as its own.
+void Withdraw(rtb200_engine* e)
+{
+    rtb200_ctx* ctx = e->ctx;
+    std::vector<rtb200_job*> part;   // jobs that hold some of their request's samples already
+    const std::vector<int> active = e->active;
+    for (int k : active) {
+        rtb200_job* j = e->owner[k];
+        CancelEntry(e, j);
+        if (j->adaptive || j->folded) part.push_back(j);
+    }
+    // Nothing is launched for jobs whose scene is gone.
+    int rc = RTB200_OK;
+    for (int k : active)
+        if (!ctx->scenes.count(e->owner[k]->scene_id)) rc = RTB200_E_INVALID;
+    const auto pending = [&] {
+        for (rtb200_job* j : part)
+            if (!JobDone(e, j->entry)) return true;
+        return false;
+    };
+    for (int step = 0; rc == RTB200_OK && step < (1 << 18) && pending(); ++step) rc = EngineStep(e, 4, false);
+    for (rtb200_job* j : part)
+        if (rc != RTB200_OK || EngineRetire(e, j) != RTB200_OK) j->spoiled = true;
+    for (int k : active) {
+        rtb200_job* j = e->owner[k];
+        if (!j) continue;   // retired
+        if (cudaMemsetAsync(j->pass, 0, 4 * (size_t)j->film_n, ctx->stream) != cudaSuccess) j->spoiled = true;
+        j->engine = nullptr;
+        j->entry = -1;
+        j->pending_spp = 0;
+    }
+}
+
 void EngineDestroy(rtb200_engine* e)
 {
     rtb200_ctx* ctx = e->ctx;
+    Withdraw(e);
     cudaStreamSynchronize(ctx->stream);
-    for (int i = 0; i < kMaxJobs; ++i)
-        if (e->owner[i]) { e->owner[i]->engine = nullptr; e->owner[i]->entry = -1; }
     DropGraph(e);
     DevFreeCached(ctx, e->buf, e->bytes);
     if (ctx->pinned.size() < kPinnedKept) ctx->pinned.push_back(e->pinned);
@@ -279,6 +321,7 @@ int EngineSubmit(rtb200_engine* e, rtb200_job* j, int spp)
     rtb200_ctx* ctx = e->ctx;
     if (spp <= 0) return SetError(ctx, RTB200_E_INVALID, "spp must be positive");
     if (j->engine) return SetError(ctx, RTB200_E_INVALID, "job is already submitted to an engine");
+    if (j->spoiled) return SetError(ctx, RTB200_E_DEVICE, "an earlier request of the job failed");
     if (j->scene->ctx != ctx) return SetError(ctx, RTB200_E_INVALID, "job and engine belong to different contexts");
     if (e->layout >= 0 && e->layout != j->scene->layout && !e->active.empty())
         return SetError(ctx, RTB200_E_INVALID, "all jobs of an engine must use the same BVH layout");
@@ -326,6 +369,7 @@ int EngineSubmit(rtb200_engine* e, rtb200_job* j, int spp)
     j->engine = e;
     j->entry = entry;
     j->pending_spp = spp;
+    j->folded = false;
     return RTB200_OK;
 }
 
@@ -405,6 +449,7 @@ int EngineStep(rtb200_engine* e, int iterations, bool graph)
     for (size_t a = 0; a < e->active.size() && err == cudaSuccess; ++a) {
         rtb200_job* j = e->owner[e->active[a]];
         if (j->pending_spp < kFoldEverySpp) continue;
+        j->folded = true;
         err = j->wide ? PtFoldWide(j->pass, j->sum, j->comp, j->wide, j->film_n, false, ctx->num_sms, st)
                       : PtFold(j->pass, j->sum, j->comp, j->film_n, ctx->num_sms, st);
     }
@@ -646,6 +691,7 @@ int rtb200_job_create(rtb200_scene* s, const rtb200_render_settings* rs, rtb200_
     rtb200_job* j = new (std::nothrow) rtb200_job();
     if (!j) return SetError(ctx, RTB200_E_OOM, "host allocation failed");
     j->scene = s;
+    j->scene_id = s->id;
     j->rs = *rs;
     j->npix = rs->width * rs->height;
     const double th = std::tan(0.5 * rs->fov_deg * 3.14159265358979323846 / 180.0);
@@ -766,6 +812,7 @@ int rtb200_job_read_film(rtb200_job* j, float* xyz)
     rtb200_ctx* ctx = j->scene->ctx;
     std::lock_guard<std::mutex> g(ctx->mu);
     if (j->engine) return SetError(ctx, RTB200_E_NOT_READY, "job has a request in flight");
+    if (j->spoiled) return SetError(ctx, RTB200_E_DEVICE, "an earlier request of the job failed");
     cudaSetDevice(ctx->device);
     // Resolved on the device into the request accumulator, which is clear
     // between requests and cleared again, so reading needs no memory.
@@ -786,6 +833,7 @@ int rtb200_job_relmse(rtb200_job* j, const float* ref_xyz, double* relmse)
     rtb200_ctx* ctx = j->scene->ctx;
     std::lock_guard<std::mutex> g(ctx->mu);
     if (j->engine) return SetError(ctx, RTB200_E_NOT_READY, "job has a request in flight");
+    if (j->spoiled) return SetError(ctx, RTB200_E_DEVICE, "an earlier request of the job failed");
     cudaSetDevice(ctx->device);
     const size_t n3 = 3 * (size_t)j->npix;
     void* buf = nullptr;
@@ -813,6 +861,7 @@ int rtb200_job_read_sample_counts(rtb200_job* j, uint32_t* counts)
     rtb200_ctx* ctx = j->scene->ctx;
     std::lock_guard<std::mutex> g(ctx->mu);
     if (j->engine) return SetError(ctx, RTB200_E_NOT_READY, "job has a request in flight");
+    if (j->spoiled) return SetError(ctx, RTB200_E_DEVICE, "an earlier request of the job failed");
     if (!j->adaptive) {
         std::fill(counts, counts + j->npix, (uint32_t)j->spp_done);
         return RTB200_OK;
@@ -829,6 +878,7 @@ int ReadColor(rtb200_job* j, double ev_mul, int tone, float* rgb, uint8_t* rgb8)
     rtb200_ctx* ctx = j->scene->ctx;
     std::lock_guard<std::mutex> g(ctx->mu);
     if (j->engine) return SetError(ctx, RTB200_E_NOT_READY, "job has a request in flight");
+    if (j->spoiled) return SetError(ctx, RTB200_E_DEVICE, "an earlier request of the job failed");
     cudaSetDevice(ctx->device);
     const size_t bytes = (rgb ? 12 : 3) * (size_t)j->npix;
     void* buf = nullptr;
