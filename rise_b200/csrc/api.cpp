@@ -137,8 +137,9 @@ cudaError_t PipelinedCast(rtb200_scene* s, const rtb200_ray* rays, int64_t n, vo
     // then pieces of 2^18, at most eight.
     constexpr int64_t kWhole = int64_t(1) << 17, kPiece = int64_t(1) << 18;
     const int64_t chunk = n <= kWhole ? n : std::max(std::min((n + 1) / 2, kPiece), (n + 7) / 8);
-    const int nbuf = n > chunk ? 2 : 1;
-    rc = EnsureStage(s, (size_t)nbuf * chunk * sizeof(rtb200_ray), (size_t)nbuf * chunk * out_bytes_per_ray);
+    // Two buffers; a second and last piece may be shorter than the first.
+    const size_t staged = (size_t)std::min(n, 2 * chunk);
+    rc = EnsureStage(s, staged * sizeof(rtb200_ray), staged * out_bytes_per_ray);
     if (rc) return cudaSuccess;
     cudaStream_t ts[2] = {ctx->stream, ctx->trace2};
     // Work counters of the two trace streams (scene scratch bytes 128 and 192).
