@@ -73,6 +73,9 @@ struct MeshBVH2 {
 void MergeMeshBVHs(const std::vector<MeshBVH2>& meshes, BuiltBVH& out);
 
 // ---- device layouts -------------------------------------------------------
+//
+// Four-wide nodes are read 32 bytes at a time (ldg8, raycast.cuh), from
+// addresses that must be multiples of 32.
 
 // FP32 wide node: 4 child boxes as SoA float4, an axis' low and high planes side
 // by side (one 32-byte load), + child links, 128 bytes.
@@ -82,7 +85,7 @@ void MergeMeshBVHs(const std::vector<MeshBVH2>& meshes, BuiltBVH& out);
 // GpuTri).  The traversal reads the first 112 bytes only (empty
 // slots are known from the link); count[i] (-1 for an empty slot) is kept
 // for the host's view of the node.
-struct alignas(16) GpuNode4 {
+struct alignas(32) GpuNode4 {
     float lox[4], hix[4];
     float loy[4], hiy[4];
     float loz[4], hiz[4];
@@ -95,7 +98,7 @@ static_assert(sizeof(GpuNode4) == 128, "GpuNode4 must be 128 bytes");
 // box = origin + q * 2^exp per axis; lower bounds are rounded down and upper
 // bounds up, and the encoder verifies the FP32 decode still contains the FP32
 // box, so culling is conservative.
-struct alignas(16) QNode4 {
+struct alignas(32) QNode4 {
     float ox, oy, oz;              // origin (min corner of the union box)
     int8_t ex, ey, ez;             // power-of-two scale exponents
     uint8_t nchild;
@@ -111,7 +114,7 @@ static_assert(sizeof(QNode4) == 64, "QNode4 must be 64 bytes");
 // each decoded box contains the FP32 box; coordinates beyond the half range
 // become -inf / +inf), the same links (kEmpty for an empty slot) and no
 // counts (leaves end at the triangle flagged last, as for GpuNode4).
-struct alignas(16) HNode4 {
+struct alignas(32) HNode4 {
     uint16_t lox[4], loy[4], loz[4];
     uint16_t hix[4], hiy[4], hiz[4];
     int32_t child[4];
