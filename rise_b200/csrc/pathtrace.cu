@@ -6,7 +6,7 @@
 // PathTracingSpectralRasterizer::IntegratePixelSpectral
 // (src/Library/Rendering/PathTracingSpectralRasterizer.cpp:121-198).
 //
-// A fixed pool of path slots lives in HBM as SoA.  One iteration is six or seven
+// A fixed pool of path slots lives in HBM as SoA.  One iteration is five to ten
 // launches over device-side queues (no host round trip):
 //   KConnect any hit for the shadow-ray queue of the iteration before;
 //            unoccluded contributions are added to the path's per-wavelength
@@ -15,11 +15,24 @@
 //            that have samples left
 //   KRegen   splat finished paths into the film, start new camera samples
 //   KExtend  closest hit for every active path (warp while-while traversal)
-//   KClassify sort the active paths by the material they hit
+//   KClassify sort the active paths by the material they hit, where scenes mix
+//            shading classes
 //   KShade   emission + MIS, next-event estimation to area lights and the
 //            sky (shadow-ray queue), hero-wavelength BSDF sampling with
-//            companion-wavelength weights, Russian roulette
-// Appends to queues are warp-aggregated (one atomic per warp).
+//            companion-wavelength weights, Russian roulette; after KClassify one
+//            launch per class
+//   KEscape  the sky's radiance for paths that left the scene (after KClassify)
+// Appends to queues are warp-aggregated (one atomic per warp and queue).
+//
+// Over deep trees (PtLaunch::coop) the paths that go on are extended on the
+// iteration's stream beside KConnect, KAssign, KRegen and the extension of the new
+// paths on a side stream: five launches for one shading class over a small tree,
+// ten for mixed ones over a deep tree.  What runs side by side shares no counter:
+// the continuing paths' KExtend reads kCntNext of the last iteration's parity and
+// feeds from trace_ctr[2 + parity], while KAssign clears kCntNext of this parity
+// and trace_ctr[0], [1] and [2 + the other parity]; the new paths' KExtend feeds
+// from trace_ctr[1], KConnect from trace_ctr[0].  The shading kernels run side by
+// side after a join and append to the same queues, with atomics.
 #include <cfloat>
 
 #include "bsdf.cuh"
@@ -605,7 +618,6 @@ __device__ __noinline__ float MeshIor(const PtScene& S, int mesh, float lam)
     return M.eta >= 0 ? Spec(S.spectra, M.eta, lam) : M.ior;
 }
 
-// The BSDF value at one wavelength for a next-event pair.
 // The shading point's spectra at its four wavelengths, looked up once: the
 // Lambertian reflectance or the GGX specular colour, the conductor's optical
 // constants and its Fresnel average for the medium around the hit.

@@ -25,8 +25,8 @@ constexpr unsigned kErrStackOverflow = 1u;
 constexpr int kEmpty = INT_MIN;      // no node / no leaf
 constexpr int kTraceBlock = 128;     // threads per block of the trace kernels
 // Traversal stack per thread: the first kTraceStack entries in shared memory
-// (20 KB per block: 8 blocks of 128 threads stay resident per SM next to 64
-// registers).  Kernels instantiated with SPILL continue it in local memory for
+// (kStackRows: 22 KB per block, 8 blocks of 128 threads stay resident per SM next
+// to 64 registers).  Kernels instantiated with SPILL continue it in local memory for
 // scenes whose TraceStackBound exceeds kTraceStack; the others carry no local
 // array at all.
 constexpr int kTraceStack = kTraceStackShared;
@@ -214,6 +214,17 @@ __device__ __forceinline__ float Min3(float a, float b, float c)
     return d;
 }
 
+// The key of child i, entered at tn if it is hit (ChildHits).
+template <bool EXACT>
+__device__ __forceinline__ int HitKey(float tn, bool hit, int i, int& link)
+{
+    if (EXACT) {
+        link = hit ? link : kEmpty;
+        return hit ? __float_as_int(tn) : kInfBits;
+    }
+    return hit ? ((__float_as_int(tn) & ~3) | i) : kMiss;
+}
+
 // Entry and exit distance of one child from the six plane offsets (plane
 // minus origin): the reference slab arithmetic (BVH.h:738-763).  The
 // reference takes min / max of the two plane distances per axis; with a
@@ -228,16 +239,6 @@ __device__ __forceinline__ float Min3(float a, float b, float c)
 // (GpuTri), and the loads and the stack below: 4,194,304 incoherent closest-hit
 // rays on a 1M-triangle soup 3810 -> 2991 us over binary16 boxes, 3909 -> 3139
 // over 8-bit and 4527 -> 4140 over FP32 ones, which are bound by L1 instead.
-template <bool EXACT>
-__device__ __forceinline__ int HitKey(float tn, bool hit, int i, int& link)
-{
-    if (EXACT) {
-        link = hit ? link : kEmpty;
-        return hit ? __float_as_int(tn) : kInfBits;
-    }
-    return hit ? ((__float_as_int(tn) & ~3) | i) : kMiss;
-}
-
 template <bool EXACT>
 __device__ __forceinline__ int SlabKey(float nx, float ny, float nz, float fx, float fy, float fz, const RayPre& p,
                                        float best, int i, bool present, int& link)
@@ -555,6 +556,7 @@ struct TraceStack {
     int* spill;
 };
 constexpr int kStackRows = kTraceStack + 4;   // and three beyond the bound
+static_assert(8 * (kStackRows * kTraceBlock * 4 + 1024) <= 228 * 1024, "8 blocks per SM");
 
 __device__ __forceinline__ void StoreShared(unsigned at, int v)
 {
@@ -988,7 +990,7 @@ __device__ __forceinline__ void IntersectW8(const WNode8* __restrict__ nodes, un
     const int e[3] = {(int)(int8_t)(em & 0xffu), (int)(int8_t)((em >> 8) & 0xffu), (int)(int8_t)((em >> 16) & 0xffu)};
     const unsigned imask = em >> 24;
     // Bounds per axis as two words of four bytes (slots 0-3, 4-7); near and
-    // far planes by the direction's sign (see SlabF32).
+    // far planes by the direction's sign (see SlabKey).
     const unsigned lo[3][2] = {{w2.x, w2.y}, {w2.z, w2.w}, {w3.x, w3.y}};
     const unsigned hi[3][2] = {{w3.z, w3.w}, {w4.x, w4.y}, {w4.z, w4.w}};
     unsigned qn[3][2], qf[3][2];
