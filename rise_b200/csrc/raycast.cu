@@ -31,7 +31,8 @@ constexpr int kCastLeaves = 2;
 // waiting for the last few to find one leaves most lanes idle.  8, 12, 14, 16 and
 // 18 lanes: closest hit of 4,194,304 incoherent rays over binary16 boxes 3314,
 // 3091, 3086, 3128, 3217 us, any hit 1649, 1543, 1524, 1548, 1581; of 100,003 rays
-// with the joint tail (COOP) 161 us with 12 and 170 with 14.
+// with the joint tail (COOP) 161 us with 12 and 170 with 14.  (Closest hits with
+// integer child keys; with whole distances 12 lanes take 2977 and 160 us.)
 template <bool ANY, bool COOP>
 constexpr int kCastLack = ANY && !COOP ? 14 : 12;
 
@@ -178,10 +179,11 @@ cudaError_t PlanFeed(K kernel, std::atomic<int>* grids, const rtb200_ctx* ctx, u
 
 // Batches of up to this many rays per SM (the resident warps' first 128 rays
 // each) use the kernels whose warps finish their last rays together.  Without
-// and with (binary16 boxes, 300k-triangle soup): 20,000 rays 164 and 87 us,
-// 100,003 255 and 167, 500,000 483 and 436, 1,000,000 (1M triangles) 916 and
-// 907; at 4,194,304 the last rays no longer count and the joint walk's code
-// costs the lane walk registers (3340 and 3505 us).
+// and with (binary16 boxes, 300k-triangle soup): 20,000 rays 155 and 105 us,
+// 100,003 245 and 160, 500,000 442 and 386.  Beyond, the last rays count for less
+// and the joint walk's registers and checks for more: 1,000,000 rays on 1M triangles
+// 821 and 789 us, 4,194,304 2975 and 2980 (any hit over 8-bit boxes 1602 and
+// 1627), and 786,432 camera rays 206 and 224.
 constexpr unsigned kCoopBatchPerSm = 4096;
 
 template <class NodeT, bool ANY, bool SPILL, bool COOP>
