@@ -518,7 +518,9 @@ KExtend(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us, in
         }
     }
     if (COOP) {
-        CoopFinish<NodeT, false, SPILL>(s, stk, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
+        const bool done = CoopFinish<NodeT, false, SPILL, !UNIFORM>(s, stk, qi >= 0, nodes, tris, ntri,
+                                                                    sstack + (threadIdx.x & ~31u), Q.err);
+        if (qi >= 0 && !done) LaneRest<NodeT, SPILL>(s, nodes, tris, ntri, stk, Q.err);
         if (qi >= 0) P.hit[slot] = make_float4(s.best, __int_as_float(s.bestSlot), s.ba, s.bb);
     }
 }
@@ -582,7 +584,7 @@ KConnect(const PtJobDev* __restrict__ jobs, PtPaths P, PtQueues Q, PtScene us)
         }
     }
     if (COOP) {
-        CoopFinish<NodeT, true, SPILL>(s, stk, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
+        CoopFinish<NodeT, true, SPILL, !UNIFORM>(s, stk, qi >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), Q.err);
         if (qi >= 0 && s.bestSlot < 0) AddShadow(P, Q.shadow[qi]);
     }
 }

@@ -32,7 +32,7 @@ constexpr int kCastLeaves = 2;
 // 18 lanes: closest hit of 4,194,304 incoherent rays over binary16 boxes 3314,
 // 3091, 3086, 3128, 3217 us, any hit 1649, 1543, 1524, 1548, 1581; of 100,003 rays
 // with the joint tail (COOP) 161 us with 12 and 170 with 14.  (Closest hits with
-// integer child keys; with whole distances 12 lanes take 2977 and 160 us.)
+// integer child keys; with whole distances 12 lanes take 2971 and 157 us.)
 template <bool ANY, bool COOP>
 constexpr int kCastLack = ANY && !COOP ? 14 : 12;
 
@@ -91,8 +91,15 @@ KTrace(const NodeT* __restrict__ nodes, const GpuTri* __restrict__ tris,
         }
     }
     if (COOP) {
-        CoopFinish<NodeT, ANY, SPILL>(s, stk, ray >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), err);
-        if (ray >= 0) StoreAnswer<ANY>(s, tris, rays, ray, hits, occ);
+        if (CoopFinish<NodeT, ANY, SPILL, false>(s, stk, ray >= 0, nodes, tris, ntri, sstack + (threadIdx.x & ~31u), err)) {
+            StoreAnswer<ANY>(s, tris, rays, ray, hits, occ);
+            ray = -1;
+        }
+        // What it left: nothing, but where triangles lie at about one distance.
+        if (!ANY && ray >= 0) {
+            LaneRest<NodeT, SPILL>(s, nodes, tris, ntri, stk, err);
+            StoreAnswer<ANY>(s, tris, rays, ray, hits, occ);
+        }
     }
 }
 
@@ -179,11 +186,10 @@ cudaError_t PlanFeed(K kernel, std::atomic<int>* grids, const rtb200_ctx* ctx, u
 
 // Batches of up to this many rays per SM (the resident warps' first 128 rays
 // each) use the kernels whose warps finish their last rays together.  Without
-// and with (binary16 boxes, 300k-triangle soup): 20,000 rays 155 and 105 us,
-// 100,003 245 and 160, 500,000 442 and 386.  Beyond, the last rays count for less
+// and with (binary16 boxes, 300k-triangle soup): 20,000 rays 155 and 85 us,
+// 100,003 245 and 157, 500,000 442 and 393.  Beyond, the last rays count for less
 // and the joint walk's registers and checks for more: 1,000,000 rays on 1M triangles
-// 821 and 789 us, 4,194,304 2975 and 2980 (any hit over 8-bit boxes 1602 and
-// 1627), and 786,432 camera rays 206 and 224.
+// 818 and 805 us, 4,194,304 2971 and 3087, 786,432 camera rays 209 and 223.
 constexpr unsigned kCoopBatchPerSm = 4096;
 
 template <class NodeT, bool ANY, bool SPILL, bool COOP>

@@ -704,32 +704,56 @@ __device__ __forceinline__ bool TraceRound(TraceState& s, const NodeT* __restric
 // node.  One step does the work of up to eight dependent steps of the lane
 // walk, so a small batch, and the end of a large one, waits for memory a few
 // times instead of once per node and triangle (1,000 rays on a 100k-triangle
-// soup: 109 -> 21 us).
+// soup: 103 -> 21 us).
 //
 // A closest hit is the lane walk's, triangle for triangle: which walk ends a ray
 // depends on its neighbours and on timing, and must not show where triangles lie
-// at one distance.  So children are ordered by the lane walk's Order, a leaf
-// waits on the stack until all nodes before it have been opened, and the hits of
-// a step are taken in the lane walk's order with its comparison.  Only boxes are
-// tested early, with a best distance that is at most too large.  Testing leaves
-// as they came gave other triangles for 1,266 of 600,000 rays on a soup whose
-// triangles lie there twice, 535 of them from run to run; the order costs 20,000
-// rays on a 300k-triangle soup 99 -> 113 us and 100,003 nothing (178 us).
+// at one distance.  The joint walk tests leaves as they come to hand, so where
+// another triangle is about as far as the nearest (kCloseUnits) it says so and leaves
+// the ray to its lane, whose walk goes on from where it was, bounded by the
+// distance found (LaneRest).  Taking any of several equal hits gave another triangle
+// to 1,266 of 600,000 rays on a soup whose triangles lie there twice, to 535 of
+// them from run to run.  Walking every ray jointly but in the lane walk's order took
+// 20,000 rays on a 300k-triangle soup 105 us; this takes 85 and any of them took 91.
+// Where all triangles lie twelve times, 20,000 rays take 269 us (any: 100, in the
+// lane walk alone 1,140).
 //
 // Everything lives in the warp's part of the stack memory: with D the deepest
 // lane stack, rows D + 1 .. D + m keep the state of the m rays, a row each,
 // and the rows above are the shared stack.
 
 // Rays left in a warp when its lanes join forces.  100,003 rays on a
-// 300k-triangle soup: 245 us without and 160 with 8 rays (3, 5 and 8 rays compared
-// with integer child keys and leaves in any order: 200, 181 and 167 us).
+// 300k-triangle soup: 245 us without and 157 with 8 rays (3, 5 and 8 rays compared
+// with integer child keys and any of equal hits: 200, 181 and 167 us).
 constexpr int kCoopRays = 8;
+
+// Triangles about as far as each other: their rounded distances are at most this
+// many units in the last place apart.  A distance T / det is rounded twice and the
+// lane walk compares products rounded once, so beyond three units (a unit is at
+// least 2^-24 of the distance) the nearer one wins in any order.  kCloseHits is as
+// much as a share or more.
+constexpr int kCloseUnits = 4;
+constexpr float kCloseHits = 1.0f / 1048576.0f;   // 2^-20
+// Share of a distance by which a box may be entered behind a triangle in it.  Both
+// are rounded: the box's entry to a few units in 2^24, the triangle's distance by
+// its barycentrics' error (2^-24 d^2 / s^2, at most 1, at distance d and size s)
+// times its extent s, at most 2^-12 d and a small factor.  Boxes are culled with
+// this much to spare, so that no triangle about as far as the best goes unseen.
+constexpr float kBoxSlack = 1.0f / 128.0f;
 
 // Words of a ray's state row.
 enum CoopWord : int {
     kCoO = 0, kCoInv = 3, kCoTmin = 6, kCoRows = 7, kCoS = 8, kCoBest = 11, kCoSlot = 12, kCoA = 13, kCoB = 14,
-    kCoNode = 15, kCoLeaf = 16, kCoSp = 17, kCoLane = 18, kCoNodes = 19, kCoTris = 21, kCoNtri = 23
+    kCoNode = 15, kCoLeaf = 16, kCoSp = 17, kCoLane = 18, kCoNodes = 19, kCoTris = 21, kCoNtri = 23,
+    kCoClose = 24, kCoAnswer = 25   // best, slot, a, b found
 };
+
+// Orders floats as integers.
+__device__ __forceinline__ int OrderedBits(float t)
+{
+    const int i = __float_as_int(t);
+    return i ^ ((i >> 31) & 0x7fffffff);
+}
 
 // Whether a warp whose lanes with `live` set still hold a ray should finish
 // them together: few rays, and room above the lane stacks for their state
@@ -797,84 +821,61 @@ __device__ __forceinline__ void CoopWalk(int* rows, int D, int m, unsigned* err)
             // Eight entries at once while that leaves a depth-first walk of one
             // entry's subtree (at most kBound more) room above them.
             const int take = max(1, min(min(8, sp), (cap - kBound - sp) / 3));
-            // Group 0 holds the top entry: lanes are in the order of the lane walk.
-            const int e = (int)group < take ? entry(sp - 1 - (int)group) : kEmpty;
+            // Group `take - 1` holds the top entry, so its children end up on top.
+            const int e = (int)group < take ? entry(sp - take + (int)group) : kEmpty;
             sp -= take;
             __syncwarp();
-            const unsigned ahead = (1u << (group * 4u)) - 1u;   // lanes of the groups before this one
-            const unsigned nodes = __ballot_sync(kFull, e >= 0);
-            int key = ANY ? kMiss : kInfBits, link = kEmpty;
-            if (e >= 0) key = Slab<NodeT>::template One<!ANY>(nd, e, (int)c, p, best, link);
-            if (ANY && key == kMiss) link = kEmpty;
-            // Four triangles of a leaf, a lane each; a longer one goes back with
-            // the rest, and leaves after it wait as they do for a node.
-            const bool leaf = e < 0 && e != kEmpty;
-            bool open = leaf && (ANY || !(nodes & ahead));
-            const int at = leaf ? ~e + (int)c : -1;
-            bool last = false, tested = false;
-            TriHit h{0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-            if (open) {
-                const TriRows r = LoadRows(tr, min(at, nt - 1), p);
-                last = __float_as_int(r.x.w) < 0 || at >= nt - 1;
-                tested = Watertight(p, r, ox, oy, oz, best, h);
-            }
-            const unsigned lasts = (__ballot_sync(kFull, last) >> (group * 4u)) & 0xfu;
-            const bool more = open && !lasts;
-            const unsigned unfinished = __ballot_sync(kFull, more);
-            if (!ANY && (unfinished & ahead)) open = false;
-            // Lanes past the leaf's last triangle looked at another leaf's.
-            tested = tested && open && !(lasts & ((1u << c) - 1u));
-            unsigned cand = __ballot_sync(kFull, tested);
-            const bool found = cand != 0u;
-            while (cand) {
-                const int from = __ffs(cand) - 1;
-                best = __shfl_sync(kFull, h.t, from);
-                const int slot = __shfl_sync(kFull, at, from);
-                const float ba = __shfl_sync(kFull, h.a, from), bb = __shfl_sync(kFull, h.b, from);
-                if (lane == 0) {
-                    word(row, kCoBest) = __float_as_int(best);
-                    word(row, kCoSlot) = slot;
-                    word(row, kCoA) = __float_as_int(ba);
-                    word(row, kCoB) = __float_as_int(bb);
+            int key = kMiss, link = kEmpty;
+            if (e >= 0)
+                key = Slab<NodeT>::template One<false>(nd, e, (int)c, p, ANY ? best : best + kBoxSlack * fabsf(best), link);
+            int at = (e < 0 && e != kEmpty) ? ~e + (int)c : -1;
+            bool found = false;
+            while (__any_sync(kFull, at >= 0)) {
+                bool last = false, hit = false;
+                TriHit h{0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+                if (at >= 0) {
+                    const TriRows r = LoadRows(tr, min(at, nt - 1), p);
+                    last = __float_as_int(r.x.w) < 0 || at >= nt - 1;
+                    hit = Watertight(p, r, ox, oy, oz, ANY ? best : best + kCloseHits * fabsf(best), h);
                 }
-                if (ANY) break;
-                cand = __ballot_sync(kFull, tested && (int)lane > from && Nearer(h, best));
+                // Lanes past the leaf's last triangle looked at another leaf's.
+                const unsigned lasts = (__ballot_sync(kFull, last) >> (group * 4u)) & 0xfu;
+                hit = hit && !(lasts & ((1u << c) - 1u));
+                const unsigned cand = __ballot_sync(kFull, hit);
+                if (cand) {
+                    const int ord = hit ? OrderedBits(h.t) : INT_MAX;
+                    const int lo = __reduce_min_sync(kFull, ord);
+                    const unsigned near = __ballot_sync(kFull, ord <= lo + kCloseUnits);
+                    const int from = __ffs(__ballot_sync(kFull, ord == lo)) - 1;
+                    if (lane == 0) word(row, kCoClose) = (near & (near - 1u)) || OrderedBits(best) <= lo + kCloseUnits;
+                    if (ANY || lo < OrderedBits(best)) {
+                        best = __shfl_sync(kFull, h.t, from);
+                        const int slot = __shfl_sync(kFull, at, from);
+                        const float ba = __shfl_sync(kFull, h.a, from), bb = __shfl_sync(kFull, h.b, from);
+                        if (lane == 0) {
+                            word(row, kCoAnswer) = __float_as_int(best);
+                            word(row, kCoAnswer + 1) = slot;
+                            word(row, kCoAnswer + 2) = __float_as_int(ba);
+                            word(row, kCoAnswer + 3) = __float_as_int(bb);
+                        }
+                    }
+                    found = true;
+                    if (ANY) break;
+                }
+                at = at >= 0 && !lasts ? at + 4 : -1;
             }
             if (ANY && found) break;
-            if (leaf && c == 0u && (!open || more)) {
-                key = 0;
-                link = open ? e - 4 : e;   // ~(first + 4)
-            }
-            // Push: a group's entries above a later group's, within a group the
-            // farther ones first.
-            const unsigned hits = __ballot_sync(kFull, link != kEmpty);
+            // Push the hit children: a lower group's below a higher group's,
+            // within a group the farther ones first.
+            const unsigned hits = __ballot_sync(kFull, key != kMiss);
             int rank = 0;
-            bool equal = false;
 #pragma unroll
-            for (unsigned x = 1; x < 4; ++x) {
+            for (int x = 1; x < 4; ++x) {
                 const int other = __shfl_xor_sync(kFull, key, x);
-                if (ANY) {
-                    rank += other != kMiss && other > key;
-                } else {
-                    rank += ((hits >> (lane ^ x)) & 1u) && __int_as_float(other) > __int_as_float(key);
-                    equal |= __int_as_float(other) == __int_as_float(key);
-                }
+                rank += other != kMiss && other > key;
             }
-            if (!ANY && __any_sync(kFull, equal && link != kEmpty)) {
-                // Children at one distance: the order is the network's.
-                ChildHits ch;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    ch.key[j] = __shfl_sync(kFull, key, (int)(lane & ~3u) + j);
-                    ch.c[j] = (hits >> ((lane & ~3u) + j)) & 1u ? j : kEmpty;
-                }
-                int k0, k1, k2, k3;
-                Order<true>(ch, k0, k1, k2, k3);
-                const int me = (int)c;
-                rank = (k3 != kEmpty && me != k3) + (k2 != kEmpty && me != k3 && me != k2) + (k1 != kEmpty && me == k0);
-            }
-            const int pos = sp + __popc((hits >> (group * 4u)) >> 4u) + rank;
-            if (link != kEmpty) {
+            const int pos = sp + __popc(hits & ((1u << (group * 4u)) - 1u)) + rank;
+            if (key != kMiss) {
                 if (pos < cap) entry(pos) = link;
                 else atomicOr(err, kErrStackOverflow);
             }
@@ -885,13 +886,15 @@ __device__ __forceinline__ void CoopWalk(int* rows, int D, int m, unsigned* err)
     }
 }
 
-// Finishes the rays of the lanes with `live` set, whose state is s and for
-// which CoopReady holds; every lane of the warp calls it.  `rows` is the
-// warp's column 0 of the stack memory.  Afterwards s.best, s.bestSlot, s.ba
-// and s.bb of the live lanes hold the result and the rest of s is undefined.
-template <class NodeT, bool ANY, bool SPILL>
-__device__ __forceinline__ void CoopFinish(TraceState& s, const TraceStack& stk, bool live, const NodeT* nodes,
-                                           const GpuTri* tris, int ntri, int* rows, unsigned* err)
+// Ends the rays of the lanes with `live` set, whose state is s and for which
+// CoopReady holds; every lane of the warp calls it.  `rows` is the warp's column 0
+// of the stack memory.  Returns whether the lane's ray is done: then s.best,
+// s.bestSlot, s.ba and s.bb hold its answer and the rest of s is undefined.  A ray
+// with several triangles about as far as the nearest is left to the lane walk, with
+// its state as it was but for a nearer bound.  OWN: lanes trace different scenes.
+template <class NodeT, bool ANY, bool SPILL, bool OWN, class NodePtr, class TriPtr>
+__device__ __forceinline__ bool CoopFinish(TraceState& s, const TraceStack& stk, bool live, NodePtr& nodes,
+                                           TriPtr& tris, int& ntri, int* rows, unsigned* err)
 {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned mask = __ballot_sync(kFull, live);
@@ -924,14 +927,101 @@ __device__ __forceinline__ void CoopFinish(TraceState& s, const TraceStack& stk,
         word(mine, kCoTris) = (int)(unsigned)(unsigned long long)tris;
         word(mine, kCoTris + 1) = (int)((unsigned long long)tris >> 32);
         word(mine, kCoNtri) = ntri;
+        word(mine, kCoClose) = 0;
+        word(mine, kCoAnswer) = __float_as_int(s.best);
+        word(mine, kCoAnswer + 1) = s.bestSlot;
+        word(mine, kCoAnswer + 2) = __float_as_int(s.ba);
+        word(mine, kCoAnswer + 3) = __float_as_int(s.bb);
     }
     __syncwarp();
     CoopWalk<NodeT, ANY, SPILL>(rows, D, m, err);
-    if (live) {
-        s.best = __int_as_float(word(mine, kCoBest));
-        s.bestSlot = word(mine, kCoSlot);
-        s.ba = __int_as_float(word(mine, kCoA));
-        s.bb = __int_as_float(word(mine, kCoB));
+    const float best = __int_as_float(word(mine, kCoAnswer));
+    if (!ANY) {
+        // The lane's state again, from its row and for every lane, so that it takes
+        // no registers meanwhile; lanes without a ray read what they never use.
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s.p.o[k] = __int_as_float(word(mine, kCoO + k));
+            s.p.inv[k] = __int_as_float(word(mine, kCoInv + k));
+        }
+        s.p.tmin = __int_as_float(word(mine, kCoTmin));
+        const int rr = word(mine, kCoRows);
+        s.p.rx = rr & 0xff; s.p.ry = (rr >> 8) & 0xff; s.p.rz = rr >> 16;
+        s.p.sx = __int_as_float(word(mine, kCoS));
+        s.p.sy = __int_as_float(word(mine, kCoS + 1));
+        s.p.sz = __int_as_float(word(mine, kCoS + 2));
+        s.node = word(mine, kCoNode);
+        s.leaf = word(mine, kCoLeaf);
+        s.sp = stk.bottom + (unsigned)word(mine, kCoSp) * kStackStep;
+        s.over = 0;
+        if (OWN) {
+            nodes = reinterpret_cast<const NodeT*>(((unsigned long long)(unsigned)word(mine, kCoNodes + 1) << 32) |
+                                                   (unsigned)word(mine, kCoNodes));
+            tris = reinterpret_cast<const GpuTri*>(((unsigned long long)(unsigned)word(mine, kCoTris + 1) << 32) |
+                                                   (unsigned)word(mine, kCoTris));
+            ntri = word(mine, kCoNtri);
+        }
+    }
+    const bool again = !ANY && word(mine, kCoClose);
+    s.best = again ? fminf(__int_as_float(word(mine, kCoBest)), best + kBoxSlack * fabsf(best)) : best;
+    s.bestSlot = word(mine, again ? kCoSlot : kCoAnswer + 1);
+    s.ba = __int_as_float(word(mine, again ? kCoA : kCoAnswer + 2));
+    s.bb = __int_as_float(word(mine, again ? kCoB : kCoAnswer + 3));
+    // Every lane has read its row before a walk that goes on overwrites it.
+    __syncwarp();
+    return live && !again;
+}
+
+// Ends the closest-hit walk of a ray that CoopFinish left, by its lane alone: the
+// lane walk without its rounds and votes, which so few rays do not need (its
+// code a second time in the kernels slowed their main loop: 100,003 rays 171 us
+// instead of 157).
+template <class NodeT, bool SPILL>
+__device__ __forceinline__ void LaneRest(TraceState& s, const NodeT* __restrict__ nodes, const GpuTri* __restrict__ tris,
+                                         int ntri, const TraceStack& stk, unsigned* err)
+{
+    const auto push = [&](int v) {
+        if (SPILL) {
+            Push(s, stk, v, err);
+        } else if (s.sp < stk.bottom + kTraceStack * kStackStep) {
+            StoreShared(s.sp, v);
+            s.sp += kStackStep;
+        } else {
+            atomicOr(err, kErrStackOverflow);
+        }
+    };
+    float ox, oy, oz;
+    PermutedOrigin(s.p, ox, oy, oz);
+    int cur = s.node;
+    if (s.leaf != kEmpty) {
+        if (cur != kEmpty) push(cur);
+        cur = s.leaf;
+    }
+    if (cur == kEmpty) cur = Pop<SPILL>(s, stk);
+    while (cur != kEmpty) {
+        if (cur >= 0) {
+            ChildHits h;
+            Slab<NodeT>::template Run<true>(nodes, cur, s.p, s.best, h);
+            int k0, k1, k2, k3;
+            Order<true>(h, k0, k1, k2, k3);
+            if (k3 != kEmpty) push(k3);
+            if (k2 != kEmpty) push(k2);
+            if (k1 != kEmpty) push(k1);
+            cur = k0 != kEmpty ? k0 : Pop<SPILL>(s, stk);
+            continue;
+        }
+        for (int slot = ~cur;; ++slot) {
+            const TriRows r = LoadRows(tris, slot, s.p);
+            TriHit hit;
+            if (Watertight(s.p, r, ox, oy, oz, s.best, hit)) {
+                s.best = hit.t;
+                s.bestSlot = slot;
+                s.ba = hit.a;
+                s.bb = hit.b;
+            }
+            if (__float_as_int(r.x.w) < 0 || slot + 1 >= ntri) break;
+        }
+        cur = Pop<SPILL>(s, stk);
     }
 }
 
