@@ -186,3 +186,43 @@ def test_small_batches_keep_the_first_triangle_met(layout, planes):
             for k in range(0, RAYS, max(n, 32)):
                 assert np.array_equal(cast(rc, rays[k:k + n])["prim"], want[k:k + n]), (n, k)
         s.close()
+
+
+def test_coincident_meshes_render_alike_alone_and_in_a_batch():
+    """Two meshes of different materials in one place: a path's hit, and so the
+    image, is the same from run to run and among other scenes' paths.  Alone
+    360,000 paths start at once, in the engine 16,384: other walks end them."""
+    from rise_b200 import pathtracer
+    descs = []
+    for k in range(2):
+        d = scenes.spheres_scene(grid=32 + 8 * k, n_spheres=4, sphere_tris=600, width=200, height=150, seed=3 + k, max_depth=6)
+        tri, meshes = d.tri9, list(d.meshes)
+        for first, count, mat, ds in meshes[:3]:
+            d.add_mesh(tri[first:first + count], (mat + 1) % len(d.materials), ds)
+        descs.append(d)
+    with raycaster.Context(0) as ctx:
+        devs = [pathtracer.upload_scene(ctx, d) for d in descs]
+
+        def job(k):
+            return pathtracer.SpectralRasterizer(ctx, descs[k], scene=devs[k])
+
+        films = []
+        for k in range(2):
+            for _ in range(3):
+                r = job(k)
+                r.rasterize_scene(12)
+                films.append((k, r.film()))
+                r.close()
+        for use_graph in (False, True):
+            eng = pathtracer.Engine(ctx, 1 << 14)
+            jobs = [job(0), job(1)]
+            eng.render(jobs, [12, 12], use_graph=use_graph)
+            films += [(k, j.film()) for k, j in enumerate(jobs)]
+            for j in jobs:
+                j.close()
+            eng.close()
+        first = {0: films[0][1], 1: films[3][1]}
+        for n, (k, f) in enumerate(films):
+            assert np.allclose(f, first[k], rtol=1e-5, atol=1e-6), n
+        for d in devs:
+            d.close()
